@@ -792,7 +792,7 @@ def long_pair_kernels(ps, per_sm=2):
     first long DNA pairs, per_sm of them per SM (one 16-warp CTA is resident
     per SM; the second pair per SM evens out the first pairs' uneven
     lengths) as far as their traceback planes fit in 40 % of the free HBM
-    (at most 120 GB): the CTA traceback fill in int16x2 lanes, then one
+    (at most 120 GB): the strip traceback fill in int16x2 lanes, then one
     walker warp per pair, timed by the batch's own events."""
     import torch
 
@@ -817,7 +817,7 @@ def long_pair_kernels(ps, per_sm=2):
     gc = sub.cells / fill_s / 1e9
     peak = dpx_cell_peak(True)
     hbm, hbm_src = hbm_peak()
-    rec = traffic_record("fill_cta16_long_dna_32")
+    rec = traffic_record("fill_strip16_long_dna_32")
     traffic = rec["dram_bytes_per_launch"] * sub.cells / rec["cells"] if rec else None
     plane_gbs = 0.5 * sub.cells / fill_s / 1e9
     # Walker bytes: the nibble of each walked cell, both gapped rows written
@@ -826,13 +826,13 @@ def long_pair_kernels(ps, per_sm=2):
     walk_bytes = float((0.5 * cols + 2 * cols).sum() + sub.a_len.sum() + sub.b_len.sum())
     return {
         "pairs": n_pairs, "cells": sub.cells,
-        "fill_cta16_kernel": {
+        "fill_strip16_kernel": {
             "fill_ms": fill_s * 1e3,
             "roofline": {"bound": "int", "achieved": gc, "peak": peak, "unit": "Gcell/s", "frac": gc / peak,
                          "traffic": traffic, "traffic_source": "ncu DRAM bytes of a 32-pair launch, scaled by cells",
                          "peak_source": "measured live: tsq_probe_dpx int16x2 rate x 2 cells / 4 DPX instructions "
                                         "per cell",
-                         "note": f"{n_pairs} pairs, one 16-warp CTA each, one CTA resident per SM"},
+                         "note": f"{n_pairs} pairs in strips of 512 rows, one warp each"},
             "plane_writes": {"bound": "hbm", "achieved": plane_gbs, "peak": hbm, "unit": "GB/s",
                              "frac": plane_gbs / hbm, "bytes_per_cell": 0.5, "peak_source": hbm_src}},
         "walk_warp_kernel": {

@@ -210,33 +210,11 @@ int align_in_waves(tsq_batch *e, const uint8_t *seqs, int64_t seqs_len, const ts
   std::vector<tsq_pair_desc> wave;
   std::vector<tsq_result> res;
   int status = TSQ_OK;
-  // Long pairs run one per CTA (the CTA fill): a wave that holds more of them
-  // than one round of resident CTAs is cut at a whole number of rounds, or
-  // its last few long pairs would start only when the first ones finish.
-  const int slots = tsq::cta_blocks(tsq::kOutTrace, p->mode == TSQ_LOCAL);
-  auto is_long = [&](int64_t k) {
-    const tsq_pair_desc &d = pairs[k];
-    return d.a_len > 0 && d.b_len > 0 && double((d.a_len + 255) / 256) * double(d.b_len + 31) > 20000.0;
-  };
   int64_t begin = 0;
   while (begin < n) {
     int64_t end = begin, used = 0;
     while (end < n && (end == begin || used + bytes[size_t(order[size_t(end)])] <= budget))
       used += bytes[size_t(order[size_t(end++)])];
-    if (slots > 0 && used <= budget) {
-      int64_t nlong = 0;
-      for (int64_t k = begin; k < end; ++k) nlong += is_long(order[size_t(k)]);
-      if (nlong > slots && nlong % slots != 0) {
-        const int64_t keep = nlong / slots * slots;
-        int64_t seen = 0, cut = end;
-        for (int64_t k = begin; k < end; ++k)
-          if (is_long(order[size_t(k)]) && seen++ == keep) {
-            cut = k;
-            break;
-          }
-        end = cut;
-      }
-    }
     if (used > budget) {  // one pair alone is larger than the budget
       for (int64_t k = begin; k < end; ++k) out[order[size_t(k)]].status = TSQ_E_TOO_LARGE;
       status = status ? status : TSQ_E_TOO_LARGE;

@@ -388,7 +388,7 @@ Shape ShapeChooser::pick(int m, int n, int rows_per_lane) const {
 void tsq_batch::release_device_buffers() {
   for (tsq::DevBuf *d : {&seqs, &codes, &pairs, &tasks, &wtasks, &res, &bnd, &planes, &plane_off, &aln, &aln_off,
                          &shape_g, &shape_r, &counters, &lut, &matrix, &overflow, &rerun_tasks, &rerun_wtasks, &ccodes,
-                         &clut, &cmatrix})
+                         &clut, &cmatrix, &strip_ws, &strip_off})
     d->release();
 }
 
@@ -414,6 +414,12 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
               int64_t call_pairs, int64_t call_cells, bool segmented);
 int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts, Scheme *sc, int *sms);
 }  // namespace
+
+// Class codes go beside the letter codes for the int16x2 fills and the strip
+// fills: every batch but local identity and forced-int32 identity.
+bool classes_needed(int out_mode, bool local, int lane) {
+  return out_mode != kOutIdent || lanes16_possible(out_mode, local, lane);
+}
 
 // int16x2 fills exist for every output but local identity.
 bool lanes16_possible(int out_mode, bool local, int lane) {
@@ -536,7 +542,7 @@ int input_prepare(tsq_batch *owner, int64_t seqs_len, const tsq_params *p, const
   int rc = prepare_object(owner, p, opts, &sc, &sms);
   if (rc) return rc;
   cudaStream_t st = owner->stream;
-  owner->classes = lanes16_possible(out_mode_of(p), p->mode == TSQ_LOCAL, p->lane);
+  owner->classes = classes_needed(out_mode_of(p), p->mode == TSQ_LOCAL, p->lane);
   owner->seqs_len = seqs_len;
   TSQ_TRY(owner->seqs.ensure(size_t(seqs_len) + 128, st, owner->async_max));
   TSQ_TRY(owner->codes.ensure(size_t(seqs_len) + 128, st, owner->async_max));
@@ -599,6 +605,60 @@ int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts
     if (!e) TSQ_TRY(cudaEventCreate(&e));
   if (!b->ev_encoded) TSQ_TRY(cudaEventCreateWithFlags(&b->ev_encoded, cudaEventDisableTiming));
   return TSQ_OK;
+}
+
+// A pair is long when its sweep on one 32-lane group takes more steps than
+// kLongSteps and kLongShare of the batch's balanced per-lane work.  Device
+// time of protein batches (log-normal lengths, median as named), shares of
+// 0.5 / 1 / 2 / 4 and no strips: 1,000 x 800 score 0.93 / 0.89 / 0.69 / 0.66 and
+// 1.53 ms, with traceback 1.91 / 1.82 / 1.57 / 1.59 and 3.27; 10,000 x 350 score
+// 0.77 / 0.77 / 0.81 / 1.16 and 1.38: below 1 short pairs pay for strips they
+// do not fill, above 2 the longest pairs on one warp are the tail.  A lone
+// warp is as fast as strips up to about 600 steps (20 pairs x 150: 0.067 ms
+// either way).  Identity output's long form is a CTA of 8 warps, worth its
+// int32 cells from 20,000 steps.
+constexpr double kLongSteps = 600.0, kLongShare = 1.5, kLongStepsCta = 20000.0;
+
+// The strip launch of the pairs at [s, e) of the sorted order: its units,
+// most work left below first (a pair's strips stay in order), the pairs'
+// records and hand-over rows.
+void plan_strips(tsq_batch *b, PlanScratch &ps, int64_t s, int64_t e, StripKind kind, std::vector<int32_t> &rsel,
+                 std::vector<int2> *units) {
+  Launch L;
+  L.strip = true;
+  L.kind = kind;
+  L.R = strip_shape(kind).R;
+  L.task_begin = int32_t(s);
+  L.n_pairs = int32_t(e - s);
+  L.wt_begin = int32_t(units->size());
+  const int rows = strip_rows(kind);
+  std::vector<SortRec> key;
+  std::vector<int2> list;
+  uint64_t most = 0;
+  int64_t entries = 0;
+  std::vector<int64_t> &off = ps.strip_off;
+  for (int64_t q = s; q < e; ++q) {
+    const int32_t k = ps.order[size_t(q)];
+    const PairDev &pd = b->pairs_h[size_t(k)];
+    rsel[size_t(k)] = L.R;
+    const int strips = std::max(1, (pd.a_len + rows - 1) / rows);
+    for (int st = 0; st < strips; ++st) {
+      const uint64_t left = uint64_t(strips - st) * uint64_t(pd.b_len + 64);
+      most = std::max(most, left);
+      key.push_back(SortRec{left, int32_t(list.size())});
+      list.push_back(make_int2(int32_t(q - s), st));
+    }
+    off.push_back(entries);
+    entries += strips > 1 ? (int64_t(pd.b_len) + 15) & ~int64_t(15) : 0;
+  }
+  for (SortRec &r : key) r.key = most - r.key;
+  radix_sort(key, ps.tmp, bit_width(most));
+  for (const SortRec &r : key) units->push_back(list[size_t(r.idx)]);
+  L.n_wtasks = int32_t(list.size());
+  const int max_blocks = strip_blocks(kind, b->out_mode, b->local, b->scheme.nclasses);
+  L.blocks = int32_t(std::min<int64_t>(max_blocks, L.n_wtasks));
+  b->strip_clear = size_t(L.n_pairs) * sizeof(StripCtl) + size_t(entries) * 8;
+  b->launches.push_back(L);
 }
 
 int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t seqs_len,
@@ -688,8 +748,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     cudaStream_t st;
     ~SyncOnExit() { cudaStreamSynchronize(st); }
   } sync_on_exit{b->stream};
-  // Batches that may run int16x2 fills also get class codes.
-  b->classes = lanes16_possible(b->out_mode, b->local, p->lane);
+  b->classes = classes_needed(b->out_mode, b->local, p->lane);
   if (!b->input_owner) {
     TSQ_TRY(b->seqs.ensure(size_t(seqs_len) + 128, b->stream, b->async_max));
     TSQ_TRY(b->codes.ensure(size_t(seqs_len) + 128, b->stream, b->async_max));
@@ -708,17 +767,17 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   // overflow-checked int16x2 kernel and are re-run in int32 if flagged;
   // everything else runs in int32.
   //
-  // Long int32 pairs go to the CTA fill (their bands striped over the 16
-  // or 8 warps of a CTA):
-  // those whose sweep on one 32-lane group -- ceil(m/256) bands of n+31
-  // steps -- would outlast the batch's balanced per-lane work (or, alone,
-  // 20,000 steps).  Under the automatic lane type, score and traceback
-  // pairs take the CTA fill in int16x2 lanes with rebased values
-  // (fill_cta16.cuh) when open + ext + max_score <= 40: the long int32
-  // pairs, and the int16x2 pairs whose sweep on one 32-lane group --
-  // ceil(m/512) passes of n+63 steps -- exceeds the same budget.
+  // Long pairs would be the batch's tail on one warp: those whose sweep on
+  // one 32-lane group -- ceil(m/256) bands of n+31 steps in int32,
+  // ceil(m/512) passes of n+63 steps in int16x2 -- outlasts the batch's
+  // balanced per-lane work (kLongShare of it, kLongSteps at least).  For score and traceback
+  // output they go to the strip fill, spread over the GPU's warps; under the
+  // automatic lane type in int16x2 lanes with rebased values (open + ext +
+  // max_score <= 40) or int32 lanes, whichever StripLoad estimates to finish
+  // first, otherwise in int32 lanes.  Long int32 identity pairs go to the CTA
+  // fill (bands striped over the 8 warps of a CTA).
   //
-  // Order: lane type (CTA int16x2, CTA int32, checked int16x2, int16x2,
+  // Order: lane type (long int16x2, long int32, checked int16x2, int16x2,
   // int32), then lane
   // width, then bands and columns descending, then input order -- one
   // 44-bit key, sorted by a stable LSD radix sort (O(n): the plan of an
@@ -762,16 +821,16 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     uint64_t buckets[3] = {0, 0, 0};  // bit (G*4 + lane type) seen
     bool bad_shape = false;
     int32_t max_bands = 0, max_cols = 0;
+    StripLoad load;
   };
   std::vector<ShapePart> sparts(8);
   {
     const double lanes = double(sms) * 24.0 * 32.0;
-    const double cta_budget = std::max(20000.0, plain ? 0.0 : double(shape_cells) / (lanes * kR));
+    const bool strips = b->out_mode != kOutIdent;
+    const double balanced = plain ? 0.0 : double(shape_cells) / (lanes * kR);
+    const double long_steps = strips ? std::max(kLongSteps, kLongShare * balanced) : std::max(kLongStepsCta, balanced);
     const bool try16 = lanes16_possible(b->out_mode, b->local, p->lane);
-    // Long pairs take the CTA fill in int16x2 lanes (rebased values) where
-    // the scheme allows it and the lane type is automatic.
-    const bool cta16 = p->lane == TSQ_LANE_AUTO && cta16_supported(b->out_mode, b->local, sc, p->gap_open,
-                                                                     p->gap_extend);
+    const bool strip16 = strips && p->lane == TSQ_LANE_AUTO && strip16_supported(sc, p->gap_open, p->gap_extend);
     parallel_for(n, [&](int64_t lo, int64_t hi, int slot) {
       ShapePart sp;
       for (int64_t k = lo; k < hi; ++k) {
@@ -787,19 +846,22 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
         }
         if (lt == 0 && pd.a_len > 0 && pd.b_len > 0) {
           const double steps32 = double((pd.a_len + 255) / 256) * double(pd.b_len + 31);
-          if (steps32 > cta_budget || ch.force.cta || (tuned && tc.cta)) lt = cta16 ? 4 : 3;
-        } else if (lt != 0 && cta16 && !ch.force.shape) {
+          if (steps32 > long_steps || ch.force.cta || (tuned && tc.cta)) lt = strip16 ? 4 : 3;
+        } else if (lt != 0 && strip16 && !ch.force.shape) {
           // An int16x2 pair whose sweep on one 32-lane group -- ceil(m/512)
           // passes of n+63 steps -- would be the batch's tail (and, when
           // checked, might need an int32 re-run on one warp as well).
           const double steps16 = double((pd.a_len + 511) / 512) * double(pd.b_len + 63);
-          if (steps16 > cta_budget) lt = 4;
+          if (steps16 > long_steps) lt = 4;
         }
         lsel[size_t(k)] = lt;
         sp.n_checked += lt == 2;
         const int rows_per_lane = (lt == 1 || lt == 2) ? 2 * kR : kR;
         Shape shp = ch.pick(pd.a_len, pd.b_len, rows_per_lane);
-        if (lt >= 3) shp = Shape{32, kR, 0};  // one 32-lane group per warp of the CTA
+        if (lt >= 3) {
+          shp = Shape{32, kR, 0};  // one 32-lane group per warp
+          if (strips) sp.load.add(pd.a_len, pd.b_len);
+        }
         shp.i16 = 0;
         if (!shape_supported(shp, b->out_mode, b->local)) sp.bad_shape = true;
         gsel[size_t(k)] = shp.G;
@@ -812,7 +874,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
         ps.cost[size_t(k)] = int64_t(bands(k)) * steps(k);
         sp.max_bands = std::max(sp.max_bands, bandk);
         sp.max_cols = std::max(sp.max_cols, colk);
-        // Ranks of the lane types 0..4, in launch order: CTA int16x2, CTA
+        // Ranks of the lane types 0..4, in launch order: long int16x2, long
         // int32, checked int16x2, int16x2, int32.
         static const uint64_t kLaneRank[5] = {4, 3, 2, 1, 0};
         // Provisional key; packed to the bits the batch needs below.
@@ -826,8 +888,10 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   int64_t n_checked = 0;
   uint64_t bucket_bits[3] = {0, 0, 0};
   int32_t max_bands = 0, max_cols = 0;
+  StripLoad load;
   for (const ShapePart &sp : sparts) {
     if (sp.bad_shape) return TSQ_E_INVALID_ARG;
+    load.merge(sp.load);
     n_checked += sp.n_checked;
     for (int w = 0; w < 3; ++w) bucket_bits[w] |= sp.buckets[w];
     max_bands = std::max(max_bands, sp.max_bands);
@@ -864,6 +928,8 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   // of warp tasks -- consecutive pairs of one lane width, 32/G per warp --
   // ordered by cost (bands x steps of the longest pair), longest first.
   b->launches.clear();
+  b->strip_clear = 0;
+  ps.strip_off.clear();
   std::vector<int2> wt_all;
   int64_t bnd_total = 0;
   int32_t checked_begin = 0;
@@ -876,20 +942,25 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
       ++e;
     }
     if (lt == 2) checked_begin = int32_t(s);
+    if (lt >= 3 && b->out_mode != kOutIdent) {
+      plan_strips(b, ps, s, e, load.pick(b->out_mode, sms, lt == 4), rsel, &wt_all);
+      if (b->launches.back().blocks <= 0) return TSQ_E_CUDA;
+      s = e;
+      continue;
+    }
     if (lt >= 3) {
       // One long pair per CTA; the CTAs pull pairs longest first.
       Launch L;
       L.R = kR;
-      L.i16 = lt == 4 ? 1 : 0;  // int16x2 lanes with rebased values
       L.cta = true;
       L.task_begin = int32_t(s);
       L.n_wtasks = int32_t(e - s);
-      const int max_blocks = lt == 4 ? cta16_blocks(b->out_mode, b->local, sc.nclasses) : cta_blocks(b->out_mode, b->local);
+      const int max_blocks = cta_blocks(b->local);
       if (max_blocks <= 0) return TSQ_E_CUDA;
       L.blocks = int32_t(std::max<int64_t>(1, std::min<int64_t>(max_blocks, e - s)));
       L.bnd_cols = ((cols + 31) / 32 + 1) * 32;
       L.bnd_offset = bnd_total;
-      bnd_total += int64_t(L.blocks) * L.bnd_cols * int64_t(cta_bnd_entry_bytes(b->out_mode));
+      bnd_total += int64_t(L.blocks) * L.bnd_cols * int64_t(cta_bnd_entry_bytes());
       bnd_total = (bnd_total + 255) & ~int64_t(255);
       b->launches.push_back(L);
       s = e;
@@ -1004,6 +1075,10 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     TSQ_TRY(b->rerun_tasks.ensure(sizeof(int32_t) * size_t(n_checked), b->stream, b->async_max));
     TSQ_TRY(b->rerun_wtasks.ensure(sizeof(int2) * size_t(n_checked), b->stream, b->async_max));
   }
+  if (b->strip_clear > 0) {
+    TSQ_TRY(b->strip_ws.ensure(b->strip_clear, b->stream, b->async_max));
+    TSQ_TRY(b->strip_off.ensure(sizeof(int64_t) * ps.strip_off.size(), b->stream, b->async_max));
+  }
   TSQ_TRY(b->rerun_h.ensure(sizeof(int32_t)));
   TSQ_TRY(b->lut.ensure(256, b->stream, b->async_max));
   TSQ_TRY(b->matrix.ensure(kLetters * kLetters, b->stream, b->async_max));
@@ -1026,6 +1101,9 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     TSQ_TRY(cudaMemcpyAsync(b->wtasks.p, wt_sorted.data(), sizeof(int2) * wt_sorted.size(), cudaMemcpyHostToDevice,
                             st));
   }
+  if (b->strip_clear > 0)
+    TSQ_TRY(cudaMemcpyAsync(b->strip_off.p, ps.strip_off.data(), sizeof(int64_t) * ps.strip_off.size(),
+                            cudaMemcpyHostToDevice, st));
   // (An input set up by input_prepare has its code tables on the device
   // already, read by encode kernels that may be running now.)
   if (!prepared) TSQ_TRY(cudaMemcpyAsync(b->lut.p, lut, 256, cudaMemcpyHostToDevice, st));
@@ -1073,8 +1151,8 @@ cudaError_t record(tsq_batch *b, int k) {
 
 // Fill launch names for the trace ranges: [i16][out_mode].
 const char *fill_range_name(const Launch &L, int out_mode) {
-  if (L.cta && L.i16) return out_mode == kOutTrace ? "fill_cta16 trace" : "fill_cta16 score";
-  if (L.cta) return out_mode == kOutTrace ? "fill_cta trace" : (out_mode == kOutIdent ? "fill_cta identity" : "fill_cta score");
+  if (L.strip) return L.kind == kStrip16 ? "fill_strip16" : "fill_strip32";
+  if (L.cta) return "fill_cta identity";
   if (L.rerun) return "fill_i32 re-run of int16 overflows";
   if (L.i16 == 1) return "fill_i16 score";
   if (L.i16 == 2) return "fill_i16 score (checked)";
@@ -1103,9 +1181,10 @@ int enqueue_run(tsq_batch *b) {
   }
   TSQ_TRY(record(b, 1));
   int32_t *rerun_count = b->counters.as<int32_t>() + nl + 1;
-  // The CTA launch (long pairs) runs on a side stream next to the others.
+  if (b->strip_clear > 0) TSQ_TRY(cudaMemsetAsync(b->strip_ws.p, 0, b->strip_clear, st));
+  // The long pairs' launch runs on a side stream next to the others.
   bool forked = false;
-  for (const Launch &L : b->launches) forked |= L.cta;
+  for (const Launch &L : b->launches) forked |= L.cta || L.strip;
   if (forked) {
     TSQ_TRY(cudaEventRecord(b->ev_fork, st));
     TSQ_TRY(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
@@ -1113,7 +1192,7 @@ int enqueue_run(tsq_batch *b) {
   for (int l = 0; l < nl; ++l) {
     const Launch &L = b->launches[size_t(l)];
     TraceRange lr(fill_range_name(L, b->out_mode));
-    if (L.cta) {
+    if (L.cta || L.strip) {
       FillArgs a{};
       a.codes = codes_dev(b);
       a.pairs = b->pairs.as<PairDev>();
@@ -1124,19 +1203,23 @@ int enqueue_run(tsq_batch *b) {
       a.gap_open = b->params.gap_open;
       a.gap_extend = b->params.gap_extend;
       a.res = b->res.as<ResultDev>();
-      a.bnd = reinterpret_cast<int32_t *>(b->bnd.as<uint8_t>() + L.bnd_offset);
-      a.bnd_cols = L.bnd_cols;
-      a.planes = b->planes.as<uint8_t>();
-      a.plane_off = b->plane_off.as<int64_t>();
       a.max_score = b->scheme.max_score;
       a.spin_limit = b->wait_polls;
-      if (L.i16) {
+      if (L.strip) {
+        a.wtasks = b->wtasks.as<int2>() + L.wt_begin;
+        a.planes = b->planes.as<uint8_t>();
+        a.plane_off = b->plane_off.as<int64_t>();
         a.ccodes = ccodes_dev(b);
         a.cmatrix = b->cmatrix.as<int8_t>();
         a.nclasses = b->scheme.nclasses;
-        TSQ_TRY(launch_cta16(b->out_mode, b->local, a, L.blocks, b->side));
+        a.strip_ctl = b->strip_ws.as<StripCtl>();
+        a.strip_rows = reinterpret_cast<uint64_t *>(a.strip_ctl + L.n_pairs);
+        a.strip_row_off = b->strip_off.as<int64_t>();
+        TSQ_TRY(launch_strip(L.kind, b->out_mode, b->local, a, L.blocks, b->side));
       } else {
-        TSQ_TRY(launch_cta(b->out_mode, b->local, a, L.blocks, b->side));
+        a.bnd = reinterpret_cast<int32_t *>(b->bnd.as<uint8_t>() + L.bnd_offset);
+        a.bnd_cols = L.bnd_cols;
+        TSQ_TRY(launch_cta(b->local, a, L.blocks, b->side));
       }
       continue;
     }
@@ -1190,6 +1273,7 @@ int enqueue_run(tsq_batch *b) {
     w.shape_G = b->shape_g.as<int32_t>();
     w.shape_R = b->shape_r.as<int32_t>();
     w.local = b->local ? 1 : 0;
+    w.emit = 1;
     w.res = b->res.as<ResultDev>();
     w.aln = b->aln.as<char>();
     w.aln_off = b->aln_off.as<int64_t>();
@@ -1425,7 +1509,7 @@ int64_t batch_device_bytes(const tsq_batch *b) {
   const tsq::DevBuf *bufs[] = {&b->seqs, &b->codes, &b->pairs, &b->tasks, &b->wtasks, &b->res, &b->bnd,
                                &b->planes, &b->plane_off, &b->aln, &b->aln_off, &b->shape_g, &b->shape_r,
                                &b->counters, &b->lut, &b->matrix, &b->overflow, &b->rerun_tasks, &b->rerun_wtasks,
-                               &b->ccodes, &b->clut, &b->cmatrix};
+                               &b->ccodes, &b->clut, &b->cmatrix, &b->strip_ws, &b->strip_off};
   int64_t total = 0;
   for (const tsq::DevBuf *d : bufs) total += int64_t(d->cap);
   return total;

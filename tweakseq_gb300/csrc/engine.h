@@ -55,6 +55,10 @@ struct Launch {
   int R = 8, i16 = 0;  // i16: 0 int32, 1 int16x2, 2 int16x2 with overflow check
   bool rerun = false;  // int32 re-run of flagged pairs (warp tasks built on the device)
   bool cta = false;    // one long pair per CTA (fill_cta.cuh); pairs tasks[task_begin, +n_wtasks)
+  bool strip = false;  // long pairs in strips (fill_strip.cu); pairs tasks[task_begin, +n_pairs), units
+                       // [wt_begin, +n_wtasks) of the warp-task list
+  StripKind kind = kStrip32;
+  int32_t n_pairs = 0;
   int32_t task_begin = 0;
   int32_t wt_begin = 0, n_wtasks = 0;  // slice of the warp-task list
   int32_t blocks = 0;
@@ -63,7 +67,7 @@ struct Launch {
 };
 
 // What the autotuner forces while it times one candidate: a lane width for
-// every pair, and (cta) the CTA fill for every int32 pair.  Carried by the
+// every pair, and (cta) the long-pair fill for every int32 pair.  Carried by the
 // batch object into its plan, so the planner's worker threads see it.
 struct TuneForce {
   bool shape = false;
@@ -73,7 +77,7 @@ struct TuneForce {
 
 // A tuned table's choice for a length bucket: lane width, lane type (i16: 1
 // int16x2 where its range is proven or checked, 0 int32) and whether int32
-// pairs take the CTA fill.
+// pairs take the long-pair fill (strips, or for identity the CTA fill).
 struct TunedChoice {
   Shape sh{};
   int cta = 0;
@@ -118,6 +122,7 @@ struct PlanScratch {
   std::vector<int8_t> s_lt;
   std::vector<int32_t> s_g, s_cols;
   std::vector<int64_t> s_cost;
+  std::vector<int64_t> strip_off;  // strip launch: each pair's first hand-over entry
 };
 
 bool tune_table_loaded();
@@ -133,7 +138,7 @@ struct tsq_batch {
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   bool capturing = false;
   cudaEvent_t ev_fetch = nullptr;  // results copied to the pinned host buffers
-  cudaStream_t side = nullptr;     // the CTA launch runs here, forked from and joined to `stream`
+  cudaStream_t side = nullptr;     // the long pairs' launch (strips or CTAs) runs here, forked from and joined to `stream`
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   tsq::Scheme scheme{};
   tsq_params params{};
@@ -141,7 +146,7 @@ struct tsq_batch {
   bool local = false;
   bool use_graph = false;
   bool autotune = false;
-  int32_t wait_polls = 0;  // CTA fill: polls per bounded wait (0 = default)
+  int32_t wait_polls = 0;  // strip and CTA fills: polls per bounded wait (0 = default)
   tsq::TuneForce tune_force;  // set by the autotuner for the next plan
   int64_t n = 0;
   int64_t seqs_len = 0;
@@ -168,6 +173,10 @@ struct tsq_batch {
 
   tsq::DevBuf seqs, codes, pairs, tasks, wtasks, res, bnd, planes, plane_off, aln, aln_off, shape_g, shape_r, counters,
       lut, matrix, overflow, rerun_tasks, rerun_wtasks;
+  // Strip fill: the pairs' records and hand-over rows (cleared before each
+  // run) and each pair's first entry in the rows.
+  tsq::DevBuf strip_ws, strip_off;
+  size_t strip_clear = 0;  // bytes of strip_ws in use
   // Score classes for the int16x2 fill (score output only).
   tsq::DevBuf ccodes, clut, cmatrix;
   bool classes = false;
@@ -234,10 +243,9 @@ int64_t cost_order(const tsq_pair_desc *pairs, int64_t n, std::vector<uint8_t> &
 // ---- per-pair rules shared by the planner and the one-pair path ----------
 // Rows per lane of every fill.
 constexpr int kFillRows = 8;
-// Longest sequence the int32 kernels take: coordinates travel in 20 bits.
-constexpr int64_t kMaxPairLen = (1 << 20) - 1;
 int out_mode_of(const tsq_params *p);
 bool lanes16_possible(int out_mode, bool local, int lane);
+bool classes_needed(int out_mode, bool local, int lane);
 // TSQ_E_INVALID_ARG for gap costs, mode, output or lane out of range.
 int check_params(const tsq_params *p);
 // TSQ_E_TOO_LARGE for a pair beyond the kernels' value and length ranges.

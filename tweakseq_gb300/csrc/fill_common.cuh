@@ -13,6 +13,7 @@ namespace fill {
 constexpr int kThreads = 128;   // 4 warps per block
 constexpr int kMatBytes = 704;  // 26*26 int8 rounded up to a 64-byte multiple
 constexpr int kAhead = 4;       // step-loop unroll
+constexpr int kSpinLimit = 1 << 22;  // polls a bounded wait makes before giving up
 
 // Compile-time flags for the step bodies.
 template <bool B>

@@ -1,11 +1,9 @@
-// fill_cta.cuh -- one long pair per CTA: the pair's row bands are striped
-// over the CTA's W warps (band b runs on warp b mod W), each warp a 32-lane
-// group of the int32 fill of fill_i32.cuh.  Consecutive bands run at the
-// same time, each a few chunks of columns behind the one above it, so a
-// pair of 50 kb sweeps with W warps instead of 1.  W is 16 where the
-// kernel fits 128 registers (global score and traceback: one CTA fills an
-// SM's 16 warps with one pair, halving a long pair's time against two
-// 8-warp CTAs), 8 otherwise (local mode, identity).
+// fill_cta.cuh -- identity output of one long pair per CTA: the pair's row
+// bands are striped over the CTA's W warps (band b runs on warp b mod W), each
+// warp a 32-lane group of the int32 identity fill of fill_i32.cuh.
+// Consecutive bands run at the same time, each a few chunks of columns behind
+// the one above it.  (Score and traceback output of long pairs run on the
+// strip fills, over the whole GPU.)
 //
 // Band-to-band rows.  The bottom row of a band is the top row of the next.
 // Between warps w and w+1 (w < W-1) it goes through a shared-memory ring of
@@ -34,21 +32,6 @@ namespace tsq {
 namespace fill {
 
 constexpr int kCtaRing = 256;               // inter-warp ring, columns (a multiple of kChunk)
-constexpr int kSpinLimit = 1 << 22;         // polls per wait before giving up
-
-template <int OUT>
-struct CtaTop {
-  using T = int2;
-};
-template <>
-struct CtaTop<kOutIdent> {
-  using T = int4;
-};
-
-// Warps per CTA for an output mode and alignment mode.
-__host__ __device__ constexpr int cta_warps(int out_mode, bool local) {
-  return (out_mode != kOutIdent && !local) ? 16 : 8;
-}
 
 // Control block after the rings: progress counters prod[W], cons[W], the
 // fail flag and two ints (task index, spare), then W reduction keys and W
@@ -56,12 +39,12 @@ __host__ __device__ constexpr int cta_warps(int out_mode, bool local) {
 __host__ __device__ constexpr int cta_keys_offset(int W) { return (4 * (2 * W + 3) + 15) & ~15; }
 __host__ __device__ constexpr int cta_ctl_bytes(int W) { return (cta_keys_offset(W) + 12 * W + 15) & ~15; }
 
-// Shared-memory bytes of the CTA fill for an output mode.
-__host__ __device__ constexpr size_t cta_smem_bytes(int out_mode, int W) {
+// Shared-memory bytes of the CTA fill.
+__host__ __device__ constexpr size_t cta_smem_bytes(int W) {
   return size_t(kMatBytes) + size_t(kLetters) * W * 32 * 8 +                           // matrix, profile
-         size_t(kTopRing) * (out_mode == kOutIdent ? 16 : 8) + kRingPad +              // warp 0's staging ring
+         size_t(kTopRing) * 16 + kRingPad +              // warp 0's staging ring
          size_t(W) * (kCodeRing + kRingPad) +                                          // code rings
-         size_t(W - 1) * kCtaRing * (out_mode == kOutIdent ? 16 : 8) +                 // inter-warp rings
+         size_t(W - 1) * kCtaRing * 16 +                 // inter-warp rings
          cta_ctl_bytes(W);                                                             // counters
 }
 
@@ -88,11 +71,11 @@ __device__ __forceinline__ bool cta_wait_geq(const volatile int *ctr, int target
   return false;
 }
 
-template <bool LOCAL, int OUT, int W>
+template <bool LOCAL, int W>
 __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
   constexpr int G = 32, R = 8, P = G * R;
   constexpr int kCtaWarps = W, kCtaThreads = W * 32;
-  using Top = typename CtaTop<OUT>::T;
+  using Top = int4;  // (H, F, path counts of H, of F)
   extern __shared__ __align__(16) uint8_t smem[];
   int8_t *s_mat = reinterpret_cast<int8_t *>(smem);
   uint2 *s_prof = reinterpret_cast<uint2 *>(smem + kMatBytes);
@@ -138,17 +121,13 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
     const bool gbad = __syncthreads_or(bad) != 0;
     const bool trivial = (m == 0 || n == 0 || gbad);
     const int passes = trivial ? 0 : (m + P - 1) / P;
-    uint8_t *planes = nullptr;
-    if constexpr (OUT == kOutTrace) planes = A.planes + A.plane_off[pid];
     if (!trivial)
       for (int j = threadIdx.x; j < n; j += blockDim.x) {
         Top v;
         v.x = edge_h(j + 1, go, ge, LOCAL);
         v.y = kNegInf;
-        if constexpr (OUT == kOutIdent) {
-          v.z = LOCAL ? 0 : j + 1;
-          v.w = 0;
-        }
+        v.z = LOCAL ? 0 : j + 1;
+        v.w = 0;
         grow[j] = v;
       }
     if (threadIdx.x < kCtaWarps) {
@@ -285,11 +264,8 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
         }
         int32_t upH = __shfl_up_sync(0xffffffffu, outH, 1);
         int32_t upF = __shfl_up_sync(0xffffffffu, outF, 1);
-        uint32_t upCH = 0, upCF = 0;
-        if constexpr (OUT == kOutIdent) {
-          upCH = __shfl_up_sync(0xffffffffu, outCH, 1);
-          upCF = __shfl_up_sync(0xffffffffu, outCF, 1);
-        }
+        uint32_t upCH = __shfl_up_sync(0xffffffffu, outCH, 1);
+        uint32_t upCF = __shfl_up_sync(0xffffffffu, outCF, 1);
         const int jj = s - t;
         const bool valid = INTERIOR || (unsigned)jj < (unsigned)n;
         const int bc = cb[k & 1];
@@ -299,10 +275,8 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
         if (t == 0) {
           upH = tv[k & 1].x;
           upF = tv[k & 1].y;
-          if constexpr (OUT == kOutIdent) {
-            upCH = uint32_t(tv[k & 1].z);
-            upCF = uint32_t(tv[k & 1].w);
-          }
+          upCH = uint32_t(tv[k & 1].z);
+          upCF = uint32_t(tv[k & 1].w);
           if (INTERIOR || jj + 1 < n) tv[(k + 1) & 1] = top_at(jj + 1);
         }
         if (valid) {
@@ -310,7 +284,6 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
           uint32_t chu = upCH, cfv = upCF, cd = cdiag;
           hdiag = upH;
           cdiag = upCH;
-          uint32_t tw = 0;
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const int32_t sc = sbyte_dyn(r < 4 ? pcur.x : pcur.y, r);
@@ -320,52 +293,27 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
             const int32_t e = max_pred(H[r] - oe, E[r] - ge, &eopen);
             const int32_t f = max_pred(hu - oe, fv - ge, &fopen);
             const int32_t dd = d + sc;
-            int32_t h;
-            if constexpr (OUT == kOutScore) {
-              h = LOCAL ? __vimax3_s32_relu(dd, e, f) : __vimax3_s32(dd, e, f);
-              if constexpr (LOCAL) {
-                if (h > best[r]) {
-                  best[r] = h;
-                  bcol[r] = jj + 1;
-                }
-              }
-            } else {
-              // H: diagonal beats E beats F on ties: pde = (diag >= E),
-              // pxf = (max(diag, E) >= F).
-              bool pde, pxf;
-              const int32_t x = max_pred(dd, e, &pde);
-              h = max_pred(x, f, &pxf);
-              int dir = pxf ? (pde ? int(kDirDiag) : int(kDirE)) : int(kDirF);
-              if (LOCAL && h <= 0) {
-                h = 0;
-                dir = kDirStop;
-              }
-              if constexpr (OUT == kOutIdent) {
-                const uint32_t ce = (eopen ? cH[r] : cE[r]) + kCol;
-                const uint32_t cfn = (fopen ? chu : cfv) + kCol;
-                const uint32_t cdd = cd + (qa[r] == bc ? kIdentCol : kCol);
-                uint32_t ch = pxf ? (pde ? cdd : ce) : cfn;
-                if (LOCAL && h <= 0) ch = 0u;
-                cd = cH[r];
-                cH[r] = ch;
-                cE[r] = ce;
-                chu = ch;
-                cfv = cfn;
-                if constexpr (LOCAL) {
-                  if (h > best[r]) {
-                    best[r] = h;
-                    bcol[r] = jj + 1;
-                    bcnt[r] = ch;
-                  }
-                }
-              } else {
-                tw |= uint32_t(dir | (eopen ? 4 : 0) | (fopen ? 8 : 0)) << (4 * r);
-                if constexpr (LOCAL) {
-                  if (h > best[r]) {
-                    best[r] = h;
-                    bcol[r] = jj + 1;
-                  }
-                }
+            // H: diagonal beats E beats F on ties: pde = (diag >= E),
+            // pxf = (max(diag, E) >= F).
+            bool pde, pxf;
+            const int32_t x = max_pred(dd, e, &pde);
+            int32_t h = max_pred(x, f, &pxf);
+            if (LOCAL) h = max(h, 0);
+            const uint32_t ce = (eopen ? cH[r] : cE[r]) + kCol;
+            const uint32_t cfn = (fopen ? chu : cfv) + kCol;
+            const uint32_t cdd = cd + (qa[r] == bc ? kIdentCol : kCol);
+            uint32_t ch = pxf ? (pde ? cdd : ce) : cfn;
+            if (LOCAL && h == 0) ch = 0u;
+            cd = cH[r];
+            cH[r] = ch;
+            cE[r] = ce;
+            chu = ch;
+            cfv = cfn;
+            if constexpr (LOCAL) {
+              if (h > best[r]) {
+                best[r] = h;
+                bcol[r] = jj + 1;
+                bcnt[r] = ch;
               }
             }
             d = H[r];
@@ -382,18 +330,12 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
             Top v;
             v.x = outH;
             v.y = outF;
-            if constexpr (OUT == kOutIdent) {
-              v.z = int32_t(outCH);
-              v.w = int32_t(outCF);
-            }
+            v.z = int32_t(outCH);
+            v.w = int32_t(outCF);
             if (w == kCtaWarps - 1)
               grow[jj] = v;
             else if (out_ring)
               out_ring[(base + jj) % kCtaRing] = v;
-          }
-          if constexpr (OUT == kOutTrace) {
-            const int64_t entry = ((int64_t)band * (n + G - 1) + s) * G + t;
-            reinterpret_cast<uint32_t *>(planes)[entry] = tw;
           }
         }
       };
@@ -473,12 +415,8 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
         o.a_end = sc > 0 ? int32_t(0xFFFFFu - uint32_t((gkey >> 20) & 0xFFFFFu)) : 0;
         o.b_end = sc > 0 ? int32_t(0xFFFFFu - uint32_t(gkey & 0xFFFFFu)) : 0;
         o.a_begin = o.b_begin = sc > 0 ? -1 : 0;
-        if (OUT == kOutIdent) {
-          o.n_ident = sc > 0 ? int32_t(cnt >> 16) : 0;
-          o.n_cols = sc > 0 ? int32_t(cnt & 0xFFFFu) : 0;
-        } else {
-          o.n_ident = o.n_cols = -1;
-        }
+        o.n_ident = sc > 0 ? int32_t(cnt >> 16) : 0;
+        o.n_cols = sc > 0 ? int32_t(cnt & 0xFFFFu) : 0;
       }
     } else {
       const int last_w = passes > 0 ? (passes - 1) % kCtaWarps : 0;
@@ -492,12 +430,12 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta_kernel(const FillArgs A) {
         o.b_end = n;
         if (m == 0 || n == 0) {
           o.score = (m + n == 0) ? 0 : -(go + (m + n) * ge);
-          o.n_ident = OUT == kOutScore ? -1 : 0;
-          o.n_cols = OUT == kOutScore ? -1 : m + n;
+          o.n_ident = 0;
+          o.n_cols = m + n;
         } else {
           o.score = last_h;
-          o.n_ident = OUT == kOutIdent ? int32_t(last_c >> 16) : -1;
-          o.n_cols = OUT == kOutIdent ? int32_t(last_c & 0xFFFFu) : -1;
+          o.n_ident = int32_t(last_c >> 16);
+          o.n_cols = int32_t(last_c & 0xFFFFu);
         }
       }
     }

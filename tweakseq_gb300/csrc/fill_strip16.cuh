@@ -1,16 +1,13 @@
-// fill_cta16.cuh -- one long pair per CTA in int16x2 lanes with rebased
-// values (global or local alignment; score or traceback output).
+// fill_strip16.cuh -- strip fill in int16x2 lanes with rebased values: strips
+// of 512 rows (score and traceback output, global or local).
 //
-// Rows go in passes of 512.  Lane t of a warp holds rows 512p + 8t .. +7
-// (band A, low halves) and 512p + 256 + 8t .. +7 (band B, high halves),
-// band B 32 steps behind band A: the cell arithmetic, decision nibbles and
-// plane layout of the int16x2 warp fill with 32 lanes per pair
-// (fill_i16.cuh).  Pass p runs on warp p mod W, and consecutive passes run
-// at the same time, each a few chunks of columns behind the one above.  The
-// passes are joined as in the int32 CTA fill (fill_cta.cuh): shared-memory
-// rings with flow control both ways between warps w and w+1, a full-width
-// row in global memory from warp W-1 back to warp 0, absolute int32 (H, F)
-// in both.
+// For long pairs that are many enough to fill the GPU, where instructions
+// per cell count.  Lane t of a warp holds rows 512p + 8t .. +7 of strip p
+// (band A, low halves) and 512p + 256 + 8t .. +7 (band B, high halves), band
+// B 32 steps behind band A: the cell arithmetic, decision nibbles and plane
+// layout of the int16x2 warp fill with 32 lanes per pair (fill_i16.cuh).
+// Strips hand their bottom rows over as fill_strip.cuh describes, as absolute
+// int32 (H, F).
 //
 // Values.  A long pair's scores leave the int16 range; the cells a warp
 // holds at one time do not.  |H(i,j) - H(i-1,j)| and |H(i,j) - H(i,j-1)|
@@ -21,87 +18,63 @@
 // 32nd step moves the base to its lane 0's first row, shifting every live
 // value by the difference (entries at minus infinity stay at the floor).
 // With open + ext + max_score <= kMaxStep16 the live values stay within
-// +-26,000 of the base.  Ring entries are converted to the warp's base as
-// lane 0 reads them, and the bottom row back to absolute values as lane 31
-// writes it.
+// +-26,000 of the base.  The top row's entries are converted to the
+// warp's base as a chunk is taken, and the bottom row back to absolute values
+// as lane 31 writes it.
 //
 // Local mode.  H's floor, 0, is -base on a warp's scale (held at the int16
 // floor when the base is higher: the live values are then all positive).
 // A local maximum may lie far from the current base, so the per-row maxima
 // of the last 32 steps are folded into one absolute (score, row, column)
 // key per lane at every move of the base, and then start again; the keys of
-// all lanes and warps give the pair's maximum, first in row-major order on
+// all lanes and strips give the pair's maximum, first in row-major order on
 // ties, as the other fills do.
-//
-// Every wait is bounded, as in the int32 CTA fill: a wait that runs out
-// marks the pair TSQ_E_TIMEOUT and makes every other wait of the CTA give
-// up, so the kernel always finishes.
 #pragma once
 
 #include <algorithm>
 #include <cstdint>
 
-#include "fill_cta.cuh"
 #include "fill_i16.cuh"
+#include "fill_strip.cuh"
 
 namespace tsq {
 namespace fill {
 
 // Largest open + ext + max_score the rebased int16x2 lanes take.
 constexpr int kMaxStep16 = 40;
+constexpr int kStripRows16 = 512;
+constexpr int kStripCols16 = 8;  // columns per hand-over chunk
 
-// Shared memory of the int16x2 CTA fill with W warps and nclasses score
-// classes.
-__host__ __device__ constexpr size_t cta16_smem_bytes(int W, int nclasses) {
-  return size_t(kMatBytes16) + size_t(2 * nclasses) * W * 32 * sizeof(uint2) +  // class matrix, profile
-         size_t(kTopRing) * sizeof(int2) + kRingPad +                           // warp 0's staging ring
-         size_t(W) * (kCodeRing16 + kRingPad) +                                 // code rings
-         size_t(W - 1) * kCtaRing * sizeof(int2) +                              // inter-warp rings
-         cta_ctl_bytes(W);                                                      // counters
+__host__ __device__ constexpr size_t strip16_smem_bytes(int nclasses) {
+  return size_t(kMatBytes16) + size_t(2 * nclasses) * 32 * sizeof(uint2) +  // class matrix, profile
+         (kTopRing + 4 + 2 * kStripCols16) * sizeof(uint32_t) +            // top ring, bottom row
+         kCodeRing16 + kRingPad;
 }
 
-// Class codes of chunk k for a warp whose top row comes from a ring: three
-// 16-byte copies by lanes 0..2, the ring's head mirrored past its end.
-__device__ __forceinline__ void stage_codes16(int k, int t, int n, const uint8_t *codes, int64_t boff,
-                                              uint8_t *code_ring) {
-  const int c0 = kChunk * k;
-  if (c0 >= n || t >= 3) return;
-  const int64_t a = ((boff + c0) & ~int64_t(15)) + 16 * t;
-  cp_async16(code_ring + (a & (kCodeRing16 - 1)), codes + a);
-  if ((a & (kCodeRing16 - 1)) == 0) cp_async16(code_ring + kCodeRing16, codes + a);
-}
-
-template <int OUT, int W, bool LOCAL>
-__global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A) {
+template <int OUT, bool LOCAL>
+__global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
   static_assert(OUT == kOutScore || OUT == kOutTrace, "score and traceback output");
-  constexpr int G = 32, R = 8, P = G * R, P2 = 2 * P;
-  constexpr int kThr = W * 32;
+  constexpr int G = 32, R = 8, P = G * R, P2 = 2 * P, C = kStripCols16;
+  constexpr int kThr = 32;
   extern __shared__ __align__(16) uint8_t smem[];
   int8_t *s_mat = reinterpret_cast<int8_t *>(smem);
   uint2 *s_prof = reinterpret_cast<uint2 *>(smem + kMatBytes16);
-  uint8_t *p = smem + kMatBytes16 + size_t(2 * A.nclasses) * kThr * sizeof(uint2);
-  int2 *stage_ring = reinterpret_cast<int2 *>(p);  // warp 0: staged global row
-  p += kTopRing * sizeof(int2) + kRingPad;
-  uint8_t *code_rings = p;
-  p += W * (kCodeRing16 + kRingPad);
-  int2 *rings = reinterpret_cast<int2 *>(p);  // ring w (w = 1..W-1) at rings + (w-1)*kCtaRing
-  p += (W - 1) * kCtaRing * sizeof(int2);
-  volatile int *prod = reinterpret_cast<volatile int *>(p);  // [W]
-  volatile int *cons = prod + W;                              // [W]
-  volatile int *fail = cons + W;
-  int *s_misc = const_cast<int *>(fail) + 1;  // task index
-  uint64_t *s_keys = reinterpret_cast<uint64_t *>(p + cta_keys_offset(W));  // [W] local maxima
-
-  for (int k = threadIdx.x; k < kMatBytes16; k += blockDim.x) {
+  const int ncls = A.nclasses;
+  // Top entries (biased H low, biased F high) on the warp's base; the first
+  // is mirrored past the end.
+  uint32_t *top_ring = reinterpret_cast<uint32_t *>(smem + kMatBytes16 + size_t(2 * ncls) * kThr * sizeof(uint2));
+  uint32_t *out_ring = top_ring + kTopRing + 4;  // the bottom row's last 2 C columns, on the warp's base
+  uint8_t *code_ring = reinterpret_cast<uint8_t *>(out_ring + 2 * C);
+  const int lane = threadIdx.x, t = lane;
+  for (int k = lane; k < kMatBytes16; k += kThr) {
     const int x = k / kMatRow16, c = k % kMatRow16;
-    s_mat[k] = (x < A.nclasses && c < A.nclasses) ? A.cmatrix[x * A.nclasses + c] : int8_t(0);
+    s_mat[k] = (x < ncls && c < ncls) ? A.cmatrix[x * ncls + c] : int8_t(0);
   }
-  // The code rings start as class 0: positions a lane reads before its
+  // The code ring starts as class 0: positions a lane reads before its
   // columns are staged (it is out of range there) index the profile.
-  for (int k = threadIdx.x; k < W * (kCodeRing16 + kRingPad); k += blockDim.x) code_rings[k] = 0;
-  __syncthreads();
+  for (int k = lane; k < kCodeRing16 + kRingPad; k += kThr) code_ring[k] = 0;
+  __syncwarp();
 
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane;
   const int32_t go = A.gap_open, ge = A.gap_extend, oe = go + ge;
   const uint32_t nge2 = pack2(-ge, -ge), noe2 = pack2(-oe, -oe);
   const uint32_t one = A.one;
@@ -110,59 +83,46 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
   const uint32_t m4 = 0u - 4u * one, m8 = 0u - 8u * one;
   const uint32_t k16 = one << 4, k256 = one << 8, k4096 = one << 12;
   (void)minus_one, (void)k1, (void)m4, (void)m8, (void)k16, (void)k256, (void)k4096;
-  int2 *grow = reinterpret_cast<int2 *>(A.bnd) + int64_t(blockIdx.x) * A.bnd_cols;  // the wrap-around row
-  uint8_t *code_ring = code_rings + w * (kCodeRing16 + kRingPad);
-  const uint2 *profA = s_prof + threadIdx.x;        // + (2c) * kThr
-  const uint2 *profB = s_prof + kThr + threadIdx.x;  // + (2c) * kThr
+  const uint2 *profA = s_prof + lane;         // + (2c) * kThr
+  const uint2 *profB = s_prof + kThr + lane;  // + (2c) * kThr
   const int src_lane = (t + G - 1) & (G - 1);        // rotate within the warp
   const uint32_t selH = t == 0 ? 0x5410u : 0x7654u;  // (top H, rotated band-A H) or the shuffled word
   const uint32_t selF = t == 0 ? 0x5432u : 0x7654u;
-  const int ncls = A.nclasses;
-  const int n_tasks = A.n_wtasks;
-  const int spin = A.spin_limit > 0 ? A.spin_limit : kSpinLimit;
 
   for (;;) {
-    if (threadIdx.x == 0) s_misc[0] = atomicAdd(A.counter, 1);
-    __syncthreads();
-    const int task = s_misc[0];
-    __syncthreads();
-    if (task >= n_tasks) break;
-    const int pid = A.tasks[task];
+    int u = 0;
+    if (lane == 0) u = atomicAdd(A.counter, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= A.n_wtasks) break;
+    const int2 unit = A.wtasks ? A.wtasks[u] : make_int2(0, u);
+    const int q = unit.x, strip = unit.y;
+    const int pid = A.tasks[q];
     const PairDev pr = A.pairs[pid];
     const int m = pr.a_len, n = pr.b_len;
     const uint8_t *qa_cls = A.ccodes + pr.a_off;
     const int64_t boff = pr.b_off;
-    bool bad = false;
-    for (int k = threadIdx.x; k < m; k += blockDim.x) bad |= A.codes[pr.a_off + k] >= kLetters;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) bad |= A.codes[boff + k] >= kLetters;
-    const bool gbad = __syncthreads_or(bad) != 0;
-    const bool trivial = (m == 0 || n == 0 || gbad);
-    const int passes = trivial ? 0 : (m + P2 - 1) / P2;
+    const int strips = max(1, (m + P2 - 1) / P2);
     const int nbands = (m + P - 1) / P;
-    uint32_t *planes = nullptr;
-    if constexpr (OUT == kOutTrace) planes = reinterpret_cast<uint32_t *>(A.planes + A.plane_off[pid]);
-    (void)planes, (void)nbands;
-    if (!trivial)
-      for (int j = threadIdx.x; j < n; j += blockDim.x) grow[j] = make_int2(edge_h(j + 1, go, ge, LOCAL), kNegInf);
-    if (threadIdx.x < W) {
-      prod[threadIdx.x] = 0;
-      cons[threadIdx.x] = 0;
-    }
-    if (threadIdx.x == 0) *fail = 0;
-    __syncthreads();
-
+    int flags = 0;
+    // Invalid residues: each strip checks its own rows, the first one also b.
+    bool bad = strip_has_bad(A.codes + pr.a_off + strip * P2, min(P2, m - strip * P2), t);
+    if (strip == 0) bad |= strip_has_bad(A.codes + boff, n, t);
+    if (__any_sync(0xffffffffu, bad)) flags = 1;
     int32_t last_h = 0;
+    int owner = -1;
     uint64_t lkey = 0;  // local: this lane's maximum so far, as (score, -row, -column)
-    const int2 *ring_in = w > 0 ? rings + (w - 1) * kCtaRing : nullptr;  // written by warp w-1
-    int2 *ring_out = w < W - 1 ? rings + w * kCtaRing : nullptr;         // read by warp w+1
 
-    for (int pass = w; pass < passes; pass += W) {
-      const int i = pass / W;  // this warp's i-th pass
-      const int base = i * n;  // cumulative column position of the pass in its rings
-      // The last pass's bottom row has no reader.
-      int2 *const out_ring = pass + 1 < passes ? ring_out : nullptr;
-      const int rowA = pass * P2 + t * R;  // band A rows rowA+1 .. rowA+R (1-based)
-      const int rowB = rowA + P;           // band B rows rowB+1 .. rowB+R
+    if (m > 0 && n > 0) {
+      const int rowA = strip * P2 + t * R;  // band A rows rowA+1 .. rowA+R (1-based)
+      const int rowB = rowA + P;            // band B rows rowB+1 .. rowB+R
+      uint32_t *planes = nullptr;
+      if constexpr (OUT == kOutTrace) planes = reinterpret_cast<uint32_t *>(A.planes + A.plane_off[pid]);
+      (void)planes, (void)nbands;
+      uint64_t *row = A.strip_rows + A.strip_row_off[q];
+      const uint32_t tag = strip_tag(strip);
+      const bool hands_down = strip + 1 < strips;
+      StripReader<C> rd{row, strip_tag(strip - 1), n, t, A.spin_limit > 0 ? A.spin_limit : kSpinLimit, false, 0u};
+      if (strip > 0) rd.ahead = rd.fetch(0);
       // Profile of this lane's 16 rows, as in the int16x2 warp fill.
       {
         int xa[R], xb[R];
@@ -196,8 +156,8 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
       }
 
       // The warp's values are relative to bw (absolute); it starts at the
-      // pass's top-left cell H(512p, 0).
-      int32_t bw = edge_h(pass * P2, go, ge, LOCAL);
+      // strip's top-left cell H(512p, 0).
+      int32_t bw = edge_h(strip * P2, go, ge, LOCAL);
       // Local: H's floor 0, and 0 - open - ext, on the warp's scale.
       uint32_t zero2 = 0u, zero_oe2 = 0u;
       auto set_zero = [&]() {
@@ -243,40 +203,49 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
       };
       uint32_t outH = kBias2, outF = kNeg2;
       const int nS = n + G - 1;
-      const int64_t wordA = ((int64_t)(2 * pass) * nS) * G + t;
-      const int64_t wordB = ((int64_t)(2 * pass + 1) * nS - G) * G + t;
-      const bool hasB = 2 * pass + 1 < nbands;
+      const int64_t wordA = ((int64_t)(2 * strip) * nS) * G + t;
+      const int64_t wordB = ((int64_t)(2 * strip + 1) * nS - G) * G + t;
+      const bool hasB = 2 * strip + 1 < nbands;
       (void)wordA, (void)wordB, (void)hasB;
 
-      // Codes (and, for warp 0, the global row's entries) of chunk c.
-      auto stage = [&](int chunk) {
-        if (w == 0) {
-          if (pass > 0) cta_wait_geq(&prod[0], (i - 1) * n + min(kChunk * (chunk + 1), n), fail, spin);
-          stage_chunk_rt<int2, kCodeRing16>(G, chunk, t, n, grow, stage_ring, A.ccodes, boff, code_ring);
-        } else {
-          stage_codes16(chunk, t, n, A.ccodes, boff, code_ring);
+      // Columns [C * chunk, C * chunk + C) of the top row, on the warp's
+      // present base, go to the ring.
+      auto take = [&](int chunk) {
+        const int col = C * chunk + t;
+        int32_t h = edge_h(col + 1, go, ge, LOCAL), f = kNegInf;
+        if (strip > 0) {
+          const uint64_t e = rd.take(chunk);
+          h = strip_h(e);
+          f = strip_f(e);
         }
+        const uint32_t word = pack2b(h - bw, max(f - bw, kNeg16));
+        if (t < C) {
+          top_ring[col & (kTopRing - 1)] = word;
+          if ((col & (kTopRing - 1)) == 0) top_ring[kTopRing] = word;
+        }
+        __syncwarp();
+      };
+      // Hands chunk `chunk` of band B's bottom row down (its columns < n),
+      // absolute.  Lane 31 puts column s - 63 at place s mod 16, so the chunk
+      // is complete after step 8 (chunk + 8) + 6, all of it on one base.
+      auto give = [&](int chunk) {
+        const int col = C * chunk + t;
+        if (hands_down && t < C && unsigned(col) < unsigned(n)) {
+          const uint32_t v = out_ring[(col - 1) & (2 * C - 1)];
+          strip_store(row + col, strip_entry(lo16b(v) + bw, hi16b(v) + bw, go + 1, tag));
+        }
+      };
+      auto stage = [&](int chunk) {
+        strip_stage_codes<kCodeRing16>(chunk, t, n, A.ccodes, boff, code_ring);
+        cp_async_commit();
       };
       cp_async_wait_all();
       __syncwarp();
       stage(0);
-      if (w > 0) cta_wait_geq(&prod[w], base + min(kChunk + 1, n), fail, spin);
-      cp_async_commit();
+      take(0);
       cp_async_wait_all();
       __syncwarp();
       stage(1);
-      cp_async_commit();
-      // Producer side: room for the first chunk of this pass's bottom row.
-      if (out_ring) cta_wait_geq(&cons[w + 1], base + kChunk - kCtaRing, fail, spin);
-
-      // Top entry of column col (absolute (H, F)) as a packed word on the
-      // warp's base: biased H low, biased F high; F may be minus infinity.
-      auto top_word = [&](int col) -> uint32_t {
-        const int2 v = w == 0 ? stage_ring[col & (kTopRing - 1)] : ring_in[(base + col) % kCtaRing];
-        const uint32_t h = uint32_t(v.x - bw + kBias16);
-        const uint32_t f = uint32_t(max(v.y - bw, kNeg16) + kBias16);
-        return imad(f, 0x10000u * one, h);
-      };
 
       uint2 pa[2], pb[2];
       uint32_t tv[2];
@@ -285,46 +254,29 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
         const int cbb = code_ring[(boff - t - G) & (kCodeRing16 - 1)];
         pa[0] = profA[(2 * ca) * kThr];
         pb[0] = profB[(2 * cbb) * kThr];
-        tv[0] = top_word(0);
+        tv[0] = top_ring[0];
       }
-      const int max_steps = n + 2 * G - 1;
-      const int steps_pad = (max_steps + 1) & ~1;
+      // (The last chunk is handed down within the padding steps.)
+      const int steps_pad = (n + 2 * G - 1 + C + 7) & ~7;
       const int i0 = min(2 * G, steps_pad);
       const int i1 = max(i0, n & ~3);
       const int cA0 = int(boff & (kCodeRing16 - 1)) - t + 1 + kCodeRing16;  // code of column jA + 1, positive
       const int cB0 = cA0 - G;                                               // code of column jB + 1
 
       auto step = [&](const int s, auto k_tag, auto interior_tag, auto last_tag, const uint8_t *codeA,
-                      const uint8_t *codeB) {
+                      const uint8_t *codeB, const uint32_t *topp, uint32_t *outp) {
         constexpr int k = decltype(k_tag)::value;
         constexpr int cur = k & 1, nxt = cur ^ 1;
         constexpr bool INTERIOR = decltype(interior_tag)::value;
         // Chunk boundaries fall on the last step of a unit only.
+        if (decltype(last_tag)::value && ((s + 1) & (C - 1)) == 0) {
+          __syncwarp();
+          give((s + 1) / C - 9);
+        }
         if (decltype(last_tag)::value && ((s + 1) & (kChunk - 1)) == 0) {
-          // Producer: publish the columns lane 31's band B finished, then
-          // wait for room for the chunk it starts.
-          const int done = min(max(s - (2 * G - 1), 0), n);
-          if (lane == G - 1) {
-            __threadfence_block();
-            if (w == W - 1)
-              prod[0] = base + done;
-            else
-              prod[w + 1] = base + done;
-          }
-          if (out_ring && done < n) cta_wait_geq(&cons[w + 1], base + done + kChunk - kCtaRing, fail, spin);
-          // Consumer: the next chunk must be there before lane 0 reads its
-          // first column; report what was read.
           cp_async_wait_all();
           __syncwarp();
           stage((s + 1) / kChunk + 1);
-          if (w > 0) {
-            if (lane == 0) {
-              __threadfence_block();  // the entries read so far are in registers
-              cons[w] = base + min(s + 2, n);
-            }
-            cta_wait_geq(&prod[w], base + min(s + 1 + kChunk + 1, n), fail, spin);
-          }
-          cp_async_commit();
           // Rebase: lane 0's first row (band A) becomes 0.  Values move by
           // -delta; entries at the floor stay there.
           // (-delta in both halves as one 32-bit addend: for delta > 0 a
@@ -358,6 +310,7 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
             sw = s;
           }
         }
+        if (decltype(last_tag)::value && ((s + 1) & (C - 1)) == 0) take((s + 1) / C);
         const uint32_t rH = __shfl_sync(0xffffffffu, outH, src_lane);
         const uint32_t rF = __shfl_sync(0xffffffffu, outF, src_lane);
         const int jA = s - t, jB = jA - G;
@@ -372,7 +325,7 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
         const uint32_t upF = prmt(tv[cur], rF, selF);
         // Lane 0's next top entry (column s + 1); every lane reads the same
         // address.
-        if (s + 1 < n) tv[nxt] = top_word(s + 1);
+        tv[nxt] = topp[k];
         const bool vA = INTERIOR || (unsigned)jA < (unsigned)n;
         const bool vB = INTERIOR || (unsigned)jB < (unsigned)n;
         if (vA || vB) {
@@ -459,14 +412,6 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
           }
           outH = H[R - 1];
           outF = fv;
-          if (t == G - 1 && vB) {
-            // Band B's bottom row, absolute, for the next pass.
-            const int2 v = make_int2(hi16b(outH) + bw, hi16b(outF) + bw);
-            if (w == W - 1)
-              grow[jB] = v;
-            else if (out_ring)
-              out_ring[(base + jB) % kCtaRing] = v;
-          }
           if constexpr (OUT == kOutTrace) {
             if constexpr (LOCAL) {
               // A local stop (H = 0) has direction 3.
@@ -477,21 +422,26 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
             if (vB && hasB) planes[wordB + (int64_t)s * G] = prmt(acc1, acc2, 0x7632u);
           }
         }
+        if (t == G - 1) outp[k] = prmt(outH, outF, 0x7632u);
       };
       int s0 = 0;
       auto pair_of_steps = [&]() {
         const uint8_t *codeA = code_ring + ((cA0 + s0) & (kCodeRing16 - 1));
         const uint8_t *codeB = code_ring + ((cB0 + s0) & (kCodeRing16 - 1));
-        step(s0, IntTag<0>{}, BoolTag<false>{}, BoolTag<false>{}, codeA, codeB);
-        step(s0 + 1, IntTag<1>{}, BoolTag<false>{}, BoolTag<true>{}, codeA, codeB);
+        const uint32_t *topp = top_ring + ((s0 & (kTopRing - 1)) + 1);
+        uint32_t *outp = out_ring + (s0 & (2 * C - 1));
+        step(s0, IntTag<0>{}, BoolTag<false>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
+        step(s0 + 1, IntTag<1>{}, BoolTag<false>{}, BoolTag<true>{}, codeA, codeB, topp, outp);
       };
       auto quad_of_steps = [&]() {
         const uint8_t *codeA = code_ring + ((cA0 + s0) & (kCodeRing16 - 1));
         const uint8_t *codeB = code_ring + ((cB0 + s0) & (kCodeRing16 - 1));
-        step(s0, IntTag<0>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB);
-        step(s0 + 1, IntTag<1>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB);
-        step(s0 + 2, IntTag<2>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB);
-        step(s0 + 3, IntTag<3>{}, BoolTag<true>{}, BoolTag<true>{}, codeA, codeB);
+        const uint32_t *topp = top_ring + ((s0 & (kTopRing - 1)) + 1);
+        uint32_t *outp = out_ring + (s0 & (2 * C - 1));
+        step(s0, IntTag<0>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
+        step(s0 + 1, IntTag<1>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
+        step(s0 + 2, IntTag<2>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
+        step(s0 + 3, IntTag<3>{}, BoolTag<true>{}, BoolTag<true>{}, codeA, codeB, topp, outp);
       };
       if constexpr (OUT == kOutScore) {
         for (; s0 < i0; s0 += 2) pair_of_steps();
@@ -502,8 +452,10 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
         auto pair_interior = [&]() {
           const uint8_t *codeA = code_ring + ((cA0 + s0) & (kCodeRing16 - 1));
           const uint8_t *codeB = code_ring + ((cB0 + s0) & (kCodeRing16 - 1));
-          step(s0, IntTag<0>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB);
-          step(s0 + 1, IntTag<1>{}, BoolTag<true>{}, BoolTag<true>{}, codeA, codeB);
+          const uint32_t *topp = top_ring + ((s0 & (kTopRing - 1)) + 1);
+        uint32_t *outp = out_ring + (s0 & (2 * C - 1));
+          step(s0, IntTag<0>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
+          step(s0 + 1, IntTag<1>{}, BoolTag<true>{}, BoolTag<true>{}, codeA, codeB, topp, outp);
         };
 #pragma unroll 1
         for (; s0 < i0; s0 += 2) pair_of_steps();
@@ -514,65 +466,23 @@ __global__ void __launch_bounds__(W * 32, 1) fill_cta16_kernel(const FillArgs A)
       }
       cp_async_wait_all();
       __syncwarp();
-      // The whole bottom row is out; everything of the input ring was read.
-      if (lane == G - 1) {
-        __threadfence_block();
-        if (w == W - 1)
-          prod[0] = base + n;
-        else
-          prod[w + 1] = base + n;
-      }
-      if (lane == 0 && w > 0) {
-        __threadfence_block();
-        cons[w] = base + n;
-      }
       fold();
-      if (!LOCAL && pass == passes - 1) {
-        const int wr = (m - 1) - pass * P2;  // row m within this pass
+      if (rd.gave_up) flags |= 2;
+      if (LOCAL) {
+        lkey = group_max<32>(lkey);
+      } else if (!hands_down) {
+        const int wr = (m - 1) - strip * P2;  // row m within this strip
         const int half = wr >= P ? 1 : 0;
         const int lr = (wr - half * P) - t * R;
+        owner = (wr % P) / R;
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (r == lr) last_h = (half ? hi16b(H[r]) : lo16b(H[r])) + bw;
       }
     }
 
-    // ---- result (every warp has finished its passes) --------------------
-    __syncthreads();
-    if constexpr (LOCAL) {
-      const uint64_t wkey = group_max<32>(lkey);
-      if (lane == 0) s_keys[w] = wkey;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint64_t gkey = 0;
-        for (int q = 0; q < W; ++q) gkey = s_keys[q] > gkey ? s_keys[q] : gkey;
-        ResultDev &o = A.res[pid];
-        o.status = gbad ? TSQ_E_INVALID_RESIDUE : (*fail ? TSQ_E_TIMEOUT : TSQ_OK);
-        const int32_t sc = int32_t(gkey >> 40);
-        o.score = sc;
-        o.a_end = sc > 0 ? int32_t(0xFFFFFu - uint32_t((gkey >> 20) & 0xFFFFFu)) : 0;
-        o.b_end = sc > 0 ? int32_t(0xFFFFFu - uint32_t(gkey & 0xFFFFFu)) : 0;
-        o.a_begin = o.b_begin = sc > 0 ? -1 : 0;
-        o.n_ident = o.n_cols = -1;
-      }
-      __syncthreads();
-      continue;
-    }
-    const int last_w = passes > 0 ? (passes - 1) % W : 0;
-    const int wr = m > 0 ? (m - 1) % P2 : 0;
-    const int owner_t = (wr % P) / R;
-    if (w == last_w && lane == owner_t) {
-      ResultDev &o = A.res[pid];
-      o.status = gbad ? TSQ_E_INVALID_RESIDUE : (*fail ? TSQ_E_TIMEOUT : TSQ_OK);
-      o.a_begin = 0;
-      o.a_end = m;
-      o.b_begin = 0;
-      o.b_end = n;
-      o.score = (m == 0 || n == 0) ? ((m + n == 0) ? 0 : -(go + (m + n) * ge)) : last_h;
-      o.n_ident = OUT == kOutScore ? -1 : (m == 0 || n == 0 ? 0 : -1);
-      o.n_cols = OUT == kOutScore ? -1 : (m == 0 || n == 0 ? m + n : -1);
-    }
-    __syncthreads();
+    strip_finish(A, q, pid, m, n, strips, t, flags, lkey, owner, last_h, LOCAL, OUT == kOutTrace);
+    __syncwarp();
   }
 }
 

@@ -30,6 +30,9 @@ constexpr uint8_t kBadCode = 0xFF;
 constexpr int kLetters = 26;
 constexpr int32_t kNegInf = -(1 << 29);  // "minus infinity" for int32 E/F
 
+// Longest sequence the int32 kernels take: coordinates travel in 20 bits.
+constexpr int64_t kMaxPairLen = (1 << 20) - 1;
+
 // Output modes of the fill kernels.
 enum : int { kOutScore = 0, kOutIdent = 1, kOutTrace = 2 };
 // Traceback nibble: bits 0-1 H source, bit 2 E opened, bit 3 F opened.
@@ -71,6 +74,16 @@ struct Shape {
 // (x = first index into the task list, y = (G << 16) | number of pairs).
 // The planner orders warp tasks longest first; warps of one persistent
 // launch pull them from a single counter.
+// What the strips of one pair leave for the one that finishes last.
+struct StripCtl {
+  uint64_t key;     // local maximum as (score, -row, -column)
+  int32_t flags;    // 1 invalid residue, 2 a wait ran out
+  int32_t done;     // strips finished
+  int32_t last_h;   // H(m, n)
+  int32_t pad[3];
+};
+static_assert(sizeof(StripCtl) == 32, "record size");
+
 struct FillArgs {
   const uint8_t *codes;
   const PairDev *pairs;
@@ -92,7 +105,13 @@ struct FillArgs {
   const uint8_t *ccodes;  // int16x2 fill: class code per residue (0 for invalid ones), same offsets as codes
   const int8_t *cmatrix;  // int16x2 fill: nclasses x nclasses class scores
   int32_t nclasses;
-  int32_t spin_limit;     // CTA fill: polls per bounded wait (0 = the compiled default)
+  int32_t spin_limit;     // CTA and strip fills: polls per bounded wait (0 = the compiled default)
+  // Strip fills (wtasks lists (position in tasks, strip); null: one pair's
+  // strips in order): per pair of the launch, a record and its hand-over row
+  // (both zero before the launch).
+  StripCtl *strip_ctl;
+  uint64_t *strip_rows;
+  const int64_t *strip_row_off;  // entries
 };
 
 // Compacts the pairs an int16 CHECK launch flagged into a warp-task list
@@ -112,6 +131,7 @@ struct WalkArgs {
   const int32_t *shape_G;  // per pair: the G and R its planes were written with
   const int32_t *shape_R;
   int32_t local;
+  int32_t emit;  // 0: counts only (no rows, no local begin coordinates)
   ResultDev *res;
   char *aln;                 // per pair: 2 * cap bytes (a row then b row)
   const int64_t *aln_off;
@@ -140,31 +160,46 @@ size_t fill_bnd_entry_bytes(int i16, int out_mode);
 cudaError_t launch_fill(int R, int i16, int out_mode, bool local, const FillArgs &a, int blocks,
                         cudaStream_t st);
 bool shape_supported(const Shape &sh, int out_mode, bool local);
-// One long pair per CTA (fill_cta.cu): FillArgs.tasks / n_wtasks hold the
-// pair list, bnd one wrap-around row of bnd_cols entries per block.
-int cta_blocks(int out_mode, bool local);
-size_t cta_bnd_entry_bytes(int out_mode);
-cudaError_t launch_cta(int out_mode, bool local, const FillArgs &a, int blocks, cudaStream_t st);
-// The same in int16x2 lanes with rebased values (fill_cta16.cu): score and
-// traceback output, global or local, open + ext + max_score <= 40.
-// FillArgs also carries the class codes, class matrix and class count.
-bool cta16_supported(int out_mode, bool local, const Scheme &sc, int32_t gap_open, int32_t gap_extend);
-int cta16_blocks(int out_mode, bool local, int nclasses);
-cudaError_t launch_cta16(int out_mode, bool local, const FillArgs &a, int blocks, cudaStream_t st);
+// One long pair per CTA (fill_cta.cu): identity output.  FillArgs.tasks /
+// n_wtasks hold the pair list, bnd one wrap-around row of bnd_cols entries
+// per block.
+int cta_blocks(bool local);
+size_t cta_bnd_entry_bytes();
+cudaError_t launch_cta(bool local, const FillArgs &a, int blocks, cudaStream_t st);
+// One pair spread over the GPU's warps in strips of rows (fill_strip.cu):
+// score and traceback output, in int32 lanes (strips of 128 rows) or int16x2
+// lanes with rebased values (512 rows; open + ext + max_score <= 40).
+// FillArgs carries the class codes, class matrix and class count, the unit
+// list and the strip workspace.
+enum StripKind : int { kStrip32 = 0, kStrip16 = 1 };
+bool strip16_supported(const Scheme &sc, int32_t gap_open, int32_t gap_extend);
+int strip_rows(StripKind kind);
+Shape strip_shape(StripKind kind);  // of the traceback planes
+int strip_blocks(StripKind kind, int out_mode, bool local, int nclasses);
+cudaError_t launch_strip(StripKind kind, int out_mode, bool local, const FillArgs &a, int blocks, cudaStream_t st);
+// The work of a set of pairs in each kind of strips, and the kind that is
+// estimated to finish first: the longer of its longest pair's chain of steps
+// and its total steps over all schedulers.
+struct StripLoad {
+  double steps[2] = {0.0, 0.0}, chain[2] = {0.0, 0.0};
+  void add(int m, int n);
+  void merge(const StripLoad &o);
+  StripKind pick(int out_mode, int sms, bool allow16) const;
+};
 cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st);
 // Residues -> letter codes and, when clut_dev / ccodes are set, score
 // classes.
 cudaError_t launch_encode(const uint8_t *seqs, int64_t len, const uint8_t *lut_dev, uint8_t *codes,
                           const uint8_t *clut_dev, uint8_t *ccodes, cudaStream_t st);
 
-// Bytes of traceback planes a pair needs under a shape.
+// Bytes of traceback planes a pair needs under a shape: words of eight cells
+// per lane, R rows (8, or 4 in int32 strips) of 8 / R steps (step = column +
+// lane).
 inline int64_t plane_bytes(int m, int n, const Shape &sh) {
   if (m <= 0 || n <= 0) return 0;
-  const int64_t P = (int64_t)sh.G * sh.R;
-  const int64_t passes = (m + P - 1) / P;
-  const int64_t entry = sh.R / 2;  // R nibbles per lane per step
-  int64_t b = passes * (int64_t)(n + sh.G - 1) * sh.G * entry;
-  return (b + 15) & ~int64_t(15);
+  const int64_t P = (int64_t)sh.G * sh.R, U = 8 / sh.R;
+  const int64_t bands = (m + P - 1) / P;
+  return (bands * ((n + sh.G - 1 + U - 1) / U) * sh.G * 4 + 15) & ~int64_t(15);
 }
 
 }  // namespace tsq

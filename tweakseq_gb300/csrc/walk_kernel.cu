@@ -23,12 +23,12 @@ namespace {
 template <class Plane, class Seq>
 __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, ResultDev &res, Plane &pl, Seq &a,
                                           Seq &b, char *out_a, char *out_b, int64_t cap, int lane) {
-  const bool writer = lane == 0;
+  const bool emit = A.emit != 0, lead = lane == 0, writer = lead && emit;
   const int m = pr.a_len, n = pr.b_len;
   int i, j;
   if (A.local) {
     if (res.score <= 0) {
-      if (writer) {
+      if (lead) {
         res.a_begin = res.a_end = res.b_begin = res.b_end = 0;
         res.n_ident = res.n_cols = 0;
       }
@@ -46,7 +46,7 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
   int ident = 0;
   for (;;) {
     if (L >= cap && (i > 0 || j > 0)) {  // cannot happen with valid planes
-      if (writer) res.status = TSQ_E_CUDA;
+      if (lead) res.status = TSQ_E_CUDA;
       return;
     }
     if (state == 0) {
@@ -70,8 +70,10 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
           if (lane < p) {
             ca = a.get(i - 1 - lane);
             cb = b.get(j - 1 - lane);
-            out_a[cap - L - 1 - lane] = char(ca);
-            out_b[cap - L - 1 - lane] = char(cb);
+            if (emit) {
+              out_a[cap - L - 1 - lane] = char(ca);
+              out_b[cap - L - 1 - lane] = char(cb);
+            }
           }
           ident += __popc(__ballot_sync(0xffffffffu, lane < p && ca == cb));
           L += p;
@@ -121,7 +123,7 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
       // An E run always ends inside the matrix (E(i,0) is minus infinity);
       // if the planes say otherwise, stop instead of leaving the matrix.
       if (j <= 0 || i <= 0) {
-        if (writer) res.status = TSQ_E_CUDA;
+        if (lead) res.status = TSQ_E_CUDA;
         return;
       }
       const int d = pl.nib(j);
@@ -135,7 +137,7 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
       if (d & 4) state = 0;
     } else {
       if (i <= 0 || j <= 0) {
-        if (writer) res.status = TSQ_E_CUDA;
+        if (lead) res.status = TSQ_E_CUDA;
         return;
       }
       const int d = pl.nib(j);
@@ -150,9 +152,11 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
       if (d & 8) state = 0;
     }
   }
-  if (!writer) return;
-  res.a_begin = i;
-  res.b_begin = j;
+  if (!lead) return;
+  if (emit || !A.local) {
+    res.a_begin = i;
+    res.b_begin = j;
+  }
   if (!A.local) {
     res.a_end = m;
     res.b_end = n;
@@ -168,53 +172,64 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
 // 0.14 ms on 2,016 protein pairs, 18.3 against 3.2 ms on 32 long DNA pairs,
 // 3.8 against 3.6 ms on 100,000 pairs.)
 constexpr int kWarpWalkWarps = 4;
-constexpr int kWS = 32, kWL = 4;  // plane window: 32 steps x 4 lanes of one band
-constexpr int kSeqWin = 128;      // residues per sequence window
+// Pairs up to which the walks leave most of the GPU idle (one warp each on
+// 152 SMs).
+constexpr int kWideWalks = 1024;
 
+// The planes of one pair, read through a window in shared memory.  Cells are
+// placed by their global lane g = (i - 1) / R (R rows per lane) and their
+// global step q = j - 1 + g, across bands; a word holds eight cells, U = 8 / R
+// steps.  The window holds WS words of steps x WL lanes: a diagonal run of c
+// cells needs c / R + 1 lanes and (c + c / R) / U + 1 words.
+template <int R, int WS, int WL>
 struct WarpPlane {
+  static constexpr int kWords = WS * WL;
+  static constexpr int kRShift = R == 8 ? 3 : 2, kUShift = 3 - kRShift;
   const uint32_t *words;
-  uint32_t *win;  // kWS * kWL words of this warp
-  int n, G, P, lane;
-  int band, t, r;
-  int wband = -1, wt = -1, ws = -1;
+  uint32_t *win;  // kWords words of this warp
+  int row_words;  // words of a band per lane
+  int gshift, lane;
+  int g = 0, r = 0;
+  int wg = -1, ws = -1;
+  static __device__ int band_words(int n, int G) { return (n + G - 1 + (1 << kUShift) - 1) >> kUShift; }
   __device__ void set_row(int i) {
-    const int row0 = i - 1;
-    band = row0 / P;
-    const int w = row0 - band * P;
-    t = w >> 3;
-    r = w & 7;
+    g = (i - 1) >> kRShift;
+    r = (i - 1) & (R - 1);
   }
   __device__ void up() {
     if (--r < 0) {
-      r = 7;
-      if (--t < 0) {
-        t = G - 1;
-        --band;
-      }
+      r = R - 1;
+      --g;
     }
   }
-  // Steps s-kWS+1..s of lanes t-kWL+1..t (clamped into the band).
+  // The nibble of row `row` at step q in its word: the row's own (R = 8), or
+  // the rows of U steps from the top down.
+  static __device__ int shift_of(int q, int row) {
+    return R == 8 ? 4 * row : 4 * (7 - ((q & ((1 << kUShift) - 1)) * R + row));
+  }
+  // Words s-WS+1..s of lanes g-WL+1..g (clamped into the planes).
   __device__ void refill(int s) {
-    wband = band;
-    wt = t;
+    wg = g;
     ws = s;
-    const int64_t row = (int64_t)band * (n + G - 1);
-    uint32_t v[kWS * kWL / 32];
+    uint32_t v[(kWords + 31) / 32];
 #pragma unroll
-    for (int q = 0; q < kWS * kWL / 32; ++q) {
+    for (int q = 0; q < (kWords + 31) / 32; ++q) {
       const int w = lane + 32 * q;
-      const int ss = max(s - w / kWL, 0), tt = max(t - w % kWL, 0);
-      v[q] = __ldg(words + (row + ss) * G + tt);
+      const int gg = max(g - w % WL, 0);
+      const int band = gg >> gshift, t = gg & ((1 << gshift) - 1);
+      const int ss = min(max(s - w / WL - ((band << gshift) >> kUShift), 0), row_words - 1);
+      v[q] = __ldg(words + ((((int64_t)band * row_words + ss) << gshift) + t));
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < kWS * kWL / 32; ++q) win[lane + 32 * q] = v[q];
+    for (int q = 0; q < (kWords + 31) / 32; ++q)
+      if (kWords % 32 == 0 || lane + 32 * q < kWords) win[lane + 32 * q] = v[q];
     __syncwarp();
   }
   __device__ int nib(int j) {
-    const int s = j - 1 + t;
-    if (band != wband || t > wt || t <= wt - kWL || s > ws || s <= ws - kWS) refill(s);
-    return int(win[(ws - s) * kWL + (wt - t)] >> (4 * r)) & 15;
+    const int q = j - 1 + g, s = q >> kUShift;
+    if (g > wg || g <= wg - WL || s > ws || s <= ws - WS) refill(s);
+    return int(win[(ws - s) * WL + (wg - g)] >> shift_of(q, r)) & 15;
   }
   // Lanes whose cell (i - lane, j - lane) lies inside the matrix and the
   // current window and takes H from the diagonal.
@@ -222,19 +237,17 @@ struct WarpPlane {
     const int ik = i - lane, jk = j - lane;
     bool d = false;
     if (ik >= 1 && jk >= 1) {
-      const int row0 = ik - 1;
-      const int bk = row0 / P;
-      const int w = row0 - bk * P;
-      const int tk = w >> 3, rk = w & 7;
-      const int sk = jk - 1 + tk;
-      if (bk == wband && tk <= wt && tk > wt - kWL && sk <= ws && sk > ws - kWS)
-        d = ((win[(ws - sk) * kWL + (wt - tk)] >> (4 * rk)) & 3) == uint32_t(kDirDiag);
+      const int gk = (ik - 1) >> kRShift, rk = (ik - 1) & (R - 1);
+      const int q = jk - 1 + gk, sk = q >> kUShift;
+      if (gk > wg - WL && sk > ws - WS)
+        d = ((win[(ws - sk) * WL + (wg - gk)] >> shift_of(q, rk)) & 3) == uint32_t(kDirDiag);
     }
     return __ballot_sync(0xffffffffu, d);
   }
 };
 
-// One sequence read backwards through a shared window of kSeqWin residues.
+// One sequence read backwards through a shared window of WIN residues.
+template <int WIN>
 struct WarpSeq {
   const uint8_t *base;
   int len;
@@ -243,46 +256,72 @@ struct WarpSeq {
   int lo = 1 << 30;
   // The window ending at idx.
   __device__ void refill_to(int idx) {
-    lo = max(0, idx - kSeqWin + 1);
-    uint8_t v[kSeqWin / 32];
+    lo = max(0, idx - WIN + 1);
+    uint8_t v[WIN / 32];
 #pragma unroll
-    for (int q = 0; q < kSeqWin / 32; ++q) {
+    for (int q = 0; q < WIN / 32; ++q) {
       const int k = lo + lane + 32 * q;
       v[q] = k < len ? base[k] : uint8_t(0);
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < kSeqWin / 32; ++q) win[lane + 32 * q] = v[q];
+    for (int q = 0; q < WIN / 32; ++q) win[lane + 32 * q] = v[q];
     __syncwarp();
   }
   __device__ uint8_t at(int idx) {
-    if (idx < lo || idx >= lo + kSeqWin) refill_to(idx);
+    if (idx < lo || idx >= lo + WIN) refill_to(idx);
     return win[idx - lo];
   }
   // Makes residues idx-31..idx (those >= 0) readable with get().
   __device__ void cover(int idx) {
-    if (max(0, idx - 31) < lo || idx >= lo + kSeqWin) refill_to(idx);
+    if (max(0, idx - 31) < lo || idx >= lo + WIN) refill_to(idx);
   }
   __device__ uint8_t get(int idx) const { return win[idx - lo]; }
 };
 
+template <int R, int WS, int WL, int WIN>
+__device__ __forceinline__ void walk_one(const WalkArgs &A, int p, uint32_t *s_plane, uint8_t (*s_seq)[WIN], int lane) {
+  using Plane = WarpPlane<R, WS, WL>;
+  const PairDev pr = A.pairs[p];
+  ResultDev &res = A.res[p];
+  WarpSeq<WIN> a{A.seqs + pr.a_off, pr.a_len, s_seq[0], lane}, b{A.seqs + pr.b_off, pr.b_len, s_seq[1], lane};
+  const int64_t cap = (int64_t)pr.a_len + pr.b_len;
+  char *out_a = A.aln + A.aln_off[p];
+  const int G = A.shape_G[p];
+  Plane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_plane,
+           Plane::band_words(pr.b_len, G), 31 - __clz(G), lane};
+  walk_pair(A, pr, res, pl, a, b, out_a, out_a + cap, cap, lane);
+}
+
+// WIDE: windows of about 48 diagonal cells and 512 residues instead of 24
+// and 128.  A refill is one memory latency whatever its size, so few pairs,
+// whose walks are a chain of refills on an idle GPU, take the wide ones; many
+// pairs, whose refills overlap, the narrow ones, which read less.
+template <bool WIDE>
 __global__ void __launch_bounds__(kWarpWalkWarps * 32) walk_warp_kernel(const WalkArgs A) {
-  __shared__ uint32_t s_plane[kWarpWalkWarps][kWS * kWL];
-  __shared__ uint8_t s_seq[kWarpWalkWarps][2][kSeqWin];
+  constexpr int WIN = WIDE ? 512 : 128;
+  constexpr int kWords = WIDE ? 576 : 182;
+  __shared__ uint32_t s_plane[kWarpWalkWarps][kWords];
+  __shared__ uint8_t s_seq[kWarpWalkWarps][2][WIN];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * kWarpWalkWarps + w;
   if (k >= A.n_tasks) return;
   const int p = A.tasks[k];
-  const PairDev pr = A.pairs[p];
-  ResultDev &res = A.res[p];
-  if (res.status != TSQ_OK) return;
-  WarpSeq a{A.seqs + pr.a_off, pr.a_len, s_seq[w][0], lane}, b{A.seqs + pr.b_off, pr.b_len, s_seq[w][1], lane};
-  const int64_t cap = (int64_t)pr.a_len + pr.b_len;
-  char *out_a = A.aln + A.aln_off[p];
-  const int G = A.shape_G[p];
-  WarpPlane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_plane[w], pr.b_len, G,
-               G * A.shape_R[p], lane};
-  walk_pair(A, pr, res, pl, a, b, out_a, out_a + cap, cap, lane);
+  if (A.res[p].status != TSQ_OK) return;
+  const int R = A.shape_R[p];
+  if constexpr (WIDE) {
+    static_assert(64 * 9 <= kWords && 32 * 14 <= kWords, "windows fit");
+    if (R == 4)
+      walk_one<4, 32, 14, WIN>(A, p, s_plane[w], s_seq[w], lane);
+    else
+      walk_one<8, 64, 9, WIN>(A, p, s_plane[w], s_seq[w], lane);
+  } else {
+    static_assert(32 * 4 <= kWords && 20 * 9 <= kWords, "windows fit");
+    if (R == 4)
+      walk_one<4, 20, 9, WIN>(A, p, s_plane[w], s_seq[w], lane);
+    else
+      walk_one<8, 32, 4, WIN>(A, p, s_plane[w], s_seq[w], lane);
+  }
 }
 
 // ASCII -> letter codes, and (when clut is set) -> score classes for the
@@ -328,7 +367,10 @@ __global__ void encode_kernel(const uint8_t *__restrict__ seqs, int64_t len, con
 cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st) {
   if (a.n_tasks <= 0) return cudaSuccess;
   const int blocks = (a.n_tasks + kWarpWalkWarps - 1) / kWarpWalkWarps;
-  walk_warp_kernel<<<blocks, kWarpWalkWarps * 32, 0, st>>>(a);
+  if (a.n_tasks <= kWideWalks)
+    walk_warp_kernel<true><<<blocks, kWarpWalkWarps * 32, 0, st>>>(a);
+  else
+    walk_warp_kernel<false><<<blocks, kWarpWalkWarps * 32, 0, st>>>(a);
   return cudaGetLastError();
 }
 
