@@ -175,3 +175,34 @@ def test_tree_bad_arguments():
     with A.Batch(ps, output="score") as b:
         b.run()
         assert L.tsq_batch_guide_tree(b._h, 5, 0, np.zeros(4, dtype=N.TREE_NODE_DTYPE).ctypes.data) == N.E_INVALID_ARG
+
+
+@pytest.mark.parametrize("method", ["upgma", "nj"])
+@pytest.mark.parametrize("kind", ["all equal", "duplicates", "negative", "1100 leaves"])
+def test_tree_rows_that_tie_or_never_settle(method, kind):
+    """Distances that leave every row open, tie most pairs, or lie below zero;
+    more rows to scan than one join keeps results of."""
+    rng = np.random.default_rng(83)
+    n = 1100 if kind == "1100 leaves" else 130
+    if kind == "all equal":
+        D = np.full((n, n), 1 << 31, dtype=np.int64)
+    elif kind == "duplicates":
+        base = np.triu(rng.integers(1 << 30, 1 << 32, (n, n)), 1)
+        g = rng.integers(0, n // 3, n)
+        D = (base + base.T)[np.ix_(g, g)]
+    else:
+        lo = -(1 << 31) if kind == "negative" else 0
+        base = np.triu(rng.integers(lo, 1 << 32, (n, n)), 1)
+        D = base + base.T
+    np.fill_diagonal(D, 0)
+    D = np.ascontiguousarray(D, dtype=np.int64)
+    _same_tree(msa.guide_tree_from_distances(D, method), O.guide_tree(D, N.TREE[method]))
+
+
+def test_tree_of_more_leaves_than_one_cluster_holds():
+    """The first joins by two launches each, the rest in one cluster."""
+    n = 3340
+    rng = np.random.default_rng(84)
+    ident, cols = _tied_identities(rng, n, levels=50)
+    want = O.guide_tree(O.identity_distances(n, ident, cols), N.TREE["upgma"])
+    _same_tree(msa.guide_tree(n, ident, cols, "upgma"), want)
