@@ -93,3 +93,31 @@ def test_invalid_residue_in_one_strip(where):
     # The cached path is usable afterwards.
     assert A.align_pair(a, b, matrix="dna", gap_open=5, gap_extend=2, output="score").score == \
         O.score(a, b, which=O.DNA, gap_open=5, gap_extend=2).score
+
+
+@pytest.mark.parametrize("local", [False, True])
+@pytest.mark.parametrize("lane", ["auto", "i16", "i32"])
+def test_identity_from_planes_equals_carried_counts(monkeypatch, local, lane):
+    """Identity output walks traceback planes where they fit in memory and
+    carries the counts through the fill where they do not: the same table
+    either way (an empty pair and an invalid residue among them), and the
+    oracle's on a sample."""
+    ps = W.uneven_pairs(n_pairs=1500, seed=74)
+    seqs, tab = A._as_inputs(ps)
+    seqs, tab = seqs.copy(), tab.copy()
+    tab["a_len"][7] = 0
+    seqs[int(tab["b_off"][9]) + 2] = ord("?")
+    pairs = (seqs, tab["a_off"], tab["a_len"], tab["b_off"], tab["b_len"])
+    kw = dict(output="identity", mode="local" if local else "global", lane=lane, check=False)
+    got = A.align_batch(pairs, **kw)
+    monkeypatch.setenv("TSQ_WAVE_BUDGET_BYTES", "1")
+    want = A.align_batch(pairs, **kw)
+    assert got.table["status"][9] == want.table["status"][9] == N.E_INVALID_RESIDUE
+    ok = np.arange(1500) != 9
+    for f in FIELDS + ("status",):
+        assert np.array_equal(got.table[f][ok], want.table[f][ok]), f
+    idx = np.arange(20, 1500, 31)
+    o = O.batch(seqs, tab["a_off"][idx], tab["a_len"][idx], tab["b_off"][idx], tab["b_len"][idx], O.BLOSUM62, 11, 1,
+                local, O.MODE_IDENT)
+    for f in ("score", "n_ident", "n_cols"):
+        assert np.array_equal(got.table[f][idx], o[f]), f

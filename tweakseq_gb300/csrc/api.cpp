@@ -88,7 +88,8 @@ int guarded(F &&f) {
 //   segments -- so a chunk waits only for the residues up to its own, and
 //   the host copies the next segment while the device fills earlier chunks.
 int align_in_chunks(ThreadCache &c, tsq_batch *e, const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *pairs,
-                    int64_t n, const tsq_params *p, const tsq_batch_opts *opts, tsq_result *out) {
+                    int64_t n, const tsq_params *p, const tsq_batch_opts *opts, tsq_result *out,
+                    bool identity_planes) {
   if (n > INT32_MAX / 2) return TSQ_E_TOO_LARGE;
   const int K = int(std::min<int64_t>(kMaxChunks, n / kChunkPairs));
   while (int(c.chunk_engines.size()) < K - 1) c.chunk_engines.emplace_back(new tsq_batch());
@@ -115,6 +116,8 @@ int align_in_chunks(ThreadCache &c, tsq_batch *e, const uint8_t *seqs, int64_t s
     c.seg_events.push_back(ev);
   }
   const tsq_batch_opts o{dev, 0, opts ? opts->autotune : 0, opts ? opts->wait_polls : 0};
+  // One way for the whole call: the chunks share their codes.
+  for (tsq_batch *x : eng) x->identity_planes = identity_planes;
 
   cudaPointerAttributes attr{};
   const bool in_place = seqs_len > 0 && cudaPointerGetAttributes(&attr, seqs) == cudaSuccess &&
@@ -369,8 +372,13 @@ int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *
       }
       if (total > budget) return align_in_waves(e, seqs, seqs_len, pairs, n, p, opts, out, bytes, budget);
     }
-    if (p && p->output != TSQ_OUT_ALIGNMENT && n >= 2 * kChunkPairs && pairs)
-      return align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out);
+    if (p && p->output != TSQ_OUT_ALIGNMENT && n >= 2 * kChunkPairs && pairs) {
+      const bool planes = tsq::identity_planes_fit(p, pairs, n);
+      const int rc = align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, planes);
+      if (rc != TSQ_E_NOMEM || !planes) return rc;
+      cudaGetLastError();
+      return align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, false);
+    }
     int rc = tsq::batch_plan(e, seqs, seqs_len, pairs, n, p, opts, false);
     if (rc) return rc;
     if ((rc = tsq::batch_run_async(e))) return rc;

@@ -409,6 +409,11 @@ tsq_batch::~tsq_batch() {
 namespace tsq {
 
 namespace {
+// What the fills compute: identity output may run on traceback planes.
+int fill_mode_of(const tsq_batch *b, const tsq_params *p) {
+  const int out = p->output == TSQ_OUT_ALIGNMENT ? kOutTrace : (p->output == TSQ_OUT_IDENTITY ? kOutIdent : kOutScore);
+  return out == kOutIdent && b->identity_planes ? kOutTrace : out;
+}
 int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t seqs_len,
               const tsq_pair_desc *pairs, int64_t n, const tsq_params *p, const tsq_batch_opts *opts, bool plain,
               int64_t call_pairs, int64_t call_cells, bool segmented);
@@ -428,6 +433,36 @@ bool lanes16_possible(int out_mode, bool local, int lane) {
 
 int out_mode_of(const tsq_params *p) {
   return p->output == TSQ_OUT_ALIGNMENT ? kOutTrace : (p->output == TSQ_OUT_IDENTITY ? kOutIdent : kOutScore);
+}
+
+// Identity output from traceback planes.  The counts ride on the path: carried
+// through the fill they cost 41 instructions per packed cell against 30 for
+// writing the decisions, and local mode has no int16x2 form of it at all, so a
+// batch whose planes fit kIdentityPlaneBytes runs the traceback fills and walks
+// them without writing rows.  (123,753 protein pairs of 250-600 residues and
+// their 498-leaf tree: 25.7 against 17.8 ms.)
+// Larger batches, and server slots (whose admission does not count planes for
+// identity), carry the counts.
+constexpr int64_t kIdentityPlaneBytes = int64_t(24) << 30;
+
+bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n) {
+  if (!p || p->output != TSQ_OUT_IDENTITY || n <= 0 || !pairs) return false;
+  int64_t budget = kIdentityPlaneBytes;
+  // (TSQ_WAVE_BUDGET_BYTES lowers it; tests use it to take the other way.)
+  if (const char *env = std::getenv("TSQ_WAVE_BUDGET_BYTES")) {
+    const long long v = std::atoll(env);
+    if (v > 0) budget = std::min<int64_t>(budget, v);
+  }
+  std::vector<int64_t> part(8, 0);
+  parallel_for(n, [&](int64_t lo, int64_t hi, int slot) {
+    int64_t sum = 0;
+    for (int64_t k = lo; k < hi && sum <= budget; ++k)
+      sum += (int64_t(std::max(pairs[k].a_len, 0)) + 255) * (int64_t(std::max(pairs[k].b_len, 0)) + 34) / 2;
+    part[size_t(slot)] = sum;
+  });
+  int64_t total = 0;
+  for (int64_t x : part) total += std::min(x, budget + 1);
+  return total <= budget;
 }
 
 int check_params(const tsq_params *p) {
@@ -501,6 +536,13 @@ int collect_one(const ResultDev &d, const char *rows, int64_t cap, tsq_result &o
 int batch_plan(tsq_batch *b, const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *pairs, int64_t n,
                const tsq_params *p, const tsq_batch_opts *opts, bool plain) {
   TraceRange tr(plain ? "plan (one pair)" : "plan");
+  if (!b) return TSQ_E_INVALID_ARG;
+  b->identity_planes = b->identity_planes_allowed && identity_planes_fit(p, pairs, n);
+  const int rc = plan_impl(b, nullptr, seqs, seqs_len, pairs, n, p, opts, plain, 0, 0, false);
+  if (rc != TSQ_E_NOMEM || !b->identity_planes) return rc;
+  cudaGetLastError();
+  b->planes.release();
+  b->identity_planes = false;
   return plan_impl(b, nullptr, seqs, seqs_len, pairs, n, p, opts, plain, 0, 0, false);
 }
 
@@ -542,7 +584,7 @@ int input_prepare(tsq_batch *owner, int64_t seqs_len, const tsq_params *p, const
   int rc = prepare_object(owner, p, opts, &sc, &sms);
   if (rc) return rc;
   cudaStream_t st = owner->stream;
-  owner->classes = classes_needed(out_mode_of(p), p->mode == TSQ_LOCAL, p->lane);
+  owner->classes = classes_needed(fill_mode_of(owner, p), p->mode == TSQ_LOCAL, p->lane);
   owner->seqs_len = seqs_len;
   TSQ_TRY(owner->seqs.ensure(size_t(seqs_len) + 128, st, owner->async_max));
   TSQ_TRY(owner->codes.ensure(size_t(seqs_len) + 128, st, owner->async_max));
@@ -572,7 +614,10 @@ namespace {
 int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts, Scheme *sc, int *sms) {
   int rc = check_params(p);
   if (rc) return rc;
-  rc = build_scheme(p, sc);
+  // (Without counts in the fill, letters that score alike share a class.)
+  tsq_params fp = *p;
+  if (fill_mode_of(b, p) == kOutTrace) fp.output = TSQ_OUT_ALIGNMENT;
+  rc = build_scheme(&fp, sc);
   if (rc) return rc;
 
   int dev = opts && opts->device >= 0 ? opts->device : -1;
@@ -655,7 +700,7 @@ void plan_strips(tsq_batch *b, PlanScratch &ps, int64_t s, int64_t e, StripKind 
   radix_sort(key, ps.tmp, bit_width(most));
   for (const SortRec &r : key) units->push_back(list[size_t(r.idx)]);
   L.n_wtasks = int32_t(list.size());
-  const int max_blocks = strip_blocks(kind, b->out_mode, b->local, b->scheme.nclasses);
+  const int max_blocks = strip_blocks(kind, b->fill_mode, b->local, b->scheme.nclasses);
   L.blocks = int32_t(std::min<int64_t>(max_blocks, L.n_wtasks));
   b->strip_clear = size_t(L.n_pairs) * sizeof(StripCtl) + size_t(entries) * 8;
   b->launches.push_back(L);
@@ -682,6 +727,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   b->scheme = sc;
   b->params = *p;
   b->out_mode = out_mode_of(p);
+  b->fill_mode = fill_mode_of(b, p);
   b->local = p->mode == TSQ_LOCAL;
   b->use_graph = opts ? opts->use_graph != 0 : false;
   b->autotune = opts ? opts->autotune != 0 : false;
@@ -748,7 +794,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     cudaStream_t st;
     ~SyncOnExit() { cudaStreamSynchronize(st); }
   } sync_on_exit{b->stream};
-  b->classes = classes_needed(b->out_mode, b->local, p->lane);
+  b->classes = classes_needed(b->fill_mode, b->local, p->lane);
   if (!b->input_owner) {
     TSQ_TRY(b->seqs.ensure(size_t(seqs_len) + 128, b->stream, b->async_max));
     TSQ_TRY(b->codes.ensure(size_t(seqs_len) + 128, b->stream, b->async_max));
@@ -826,10 +872,10 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   std::vector<ShapePart> sparts(8);
   {
     const double lanes = double(sms) * 24.0 * 32.0;
-    const bool strips = b->out_mode != kOutIdent;
+    const bool strips = b->fill_mode != kOutIdent;
     const double balanced = plain ? 0.0 : double(shape_cells) / (lanes * kR);
     const double long_steps = strips ? std::max(kLongSteps, kLongShare * balanced) : std::max(kLongStepsCta, balanced);
-    const bool try16 = lanes16_possible(b->out_mode, b->local, p->lane);
+    const bool try16 = lanes16_possible(b->fill_mode, b->local, p->lane);
     const bool strip16 = strips && p->lane == TSQ_LANE_AUTO && strip16_supported(sc, p->gap_open, p->gap_extend);
     parallel_for(n, [&](int64_t lo, int64_t hi, int slot) {
       ShapePart sp;
@@ -863,7 +909,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
           if (strips) sp.load.add(pd.a_len, pd.b_len);
         }
         shp.i16 = 0;
-        if (!shape_supported(shp, b->out_mode, b->local)) sp.bad_shape = true;
+        if (!shape_supported(shp, b->fill_mode, b->local)) sp.bad_shape = true;
         gsel[size_t(k)] = shp.G;
         rsel[size_t(k)] = shp.R;
         const int bit = shp.G * 4 + lt;
@@ -942,8 +988,8 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
       ++e;
     }
     if (lt == 2) checked_begin = int32_t(s);
-    if (lt >= 3 && b->out_mode != kOutIdent) {
-      plan_strips(b, ps, s, e, load.pick(b->out_mode, sms, lt == 4), rsel, &wt_all);
+    if (lt >= 3 && b->fill_mode != kOutIdent) {
+      plan_strips(b, ps, s, e, load.pick(b->fill_mode, sms, lt == 4), rsel, &wt_all);
       if (b->launches.back().blocks <= 0) return TSQ_E_CUDA;
       s = e;
       continue;
@@ -997,7 +1043,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     L.wt_begin = int32_t(wt_all.size());
     L.n_wtasks = int32_t(wt.size());
     for (int32_t w : worder) wt_all.push_back(wt[size_t(w)]);
-    const int max_blocks = fill_blocks(L.R, L.i16, b->out_mode, b->local, sc.nclasses);
+    const int max_blocks = fill_blocks(L.R, L.i16, b->fill_mode, b->local, sc.nclasses);
     if (max_blocks <= 0) return TSQ_E_CUDA;
     const int warps_per_block = fill_threads_for(L.i16) / 32;
     const int64_t needed = (int64_t(L.n_wtasks) + warps_per_block - 1) / warps_per_block;
@@ -1006,7 +1052,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     L.bnd_cols = ((cols + 31) / 32 + 1) * 32;
     L.bnd_offset = bnd_total;
     bnd_total += int64_t(L.blocks) * warps_per_block * 8 * L.bnd_cols *
-                 int64_t(fill_bnd_entry_bytes(L.i16, b->out_mode));
+                 int64_t(fill_bnd_entry_bytes(L.i16, b->fill_mode));
     bnd_total = (bnd_total + 255) & ~int64_t(255);
     b->launches.push_back(L);
     s = e;
@@ -1023,19 +1069,19 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     L.R = kR;
     L.i16 = 0;
     L.rerun = true;
-    const int max_blocks = fill_blocks(L.R, 0, b->out_mode, b->local);
+    const int max_blocks = fill_blocks(L.R, 0, b->fill_mode, b->local);
     if (max_blocks <= 0) return TSQ_E_CUDA;
     const int warps_per_block = fill_threads_for(0) / 32;
     L.blocks = int32_t(std::max<int64_t>(1, std::min<int64_t>(max_blocks, (n_checked + warps_per_block - 1) /
                                                                              warps_per_block)));
     L.bnd_cols = ((cols + 31) / 32 + 1) * 32;
     L.bnd_offset = bnd_total;
-    bnd_total += int64_t(L.blocks) * warps_per_block * 8 * L.bnd_cols * int64_t(fill_bnd_entry_bytes(0, b->out_mode));
+    bnd_total += int64_t(L.blocks) * warps_per_block * 8 * L.bnd_cols * int64_t(fill_bnd_entry_bytes(0, b->fill_mode));
     b->launches.push_back(L);
   }
   b->stats.pairs = n;
   b->stats.cells = cells;
-  b->stats.launches = int32_t(b->launches.size()) + 1 + (b->out_mode == kOutTrace ? 1 : 0) + (n_checked > 0 ? 1 : 0);
+  b->stats.launches = int32_t(b->launches.size()) + 1 + (b->fill_mode == kOutTrace ? 1 : 0) + (n_checked > 0 ? 1 : 0);
   b->stats.buckets = __builtin_popcountll(bucket_bits[0]) + __builtin_popcountll(bucket_bits[1]) +
                       __builtin_popcountll(bucket_bits[2]);
   const std::vector<int2> &wt_sorted = wt_all;
@@ -1045,13 +1091,18 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   b->aln_off_h.clear();
   b->aln_bytes = 0;
   int64_t plane_total = 0;
-  if (b->out_mode == kOutTrace) {
+  if (b->fill_mode == kOutTrace) {
     ploff.resize(size_t(n));
-    b->aln_off_h.resize(size_t(n));
     for (int64_t k = 0; k < n; ++k) {
       const PairDev &pd = b->pairs_h[size_t(k)];
       ploff[size_t(k)] = plane_total;
       plane_total += plane_bytes(pd.a_len, pd.b_len, Shape{gsel[size_t(k)], rsel[size_t(k)], 0});
+    }
+  }
+  if (b->out_mode == kOutTrace) {
+    b->aln_off_h.resize(size_t(n));
+    for (int64_t k = 0; k < n; ++k) {
+      const PairDev &pd = b->pairs_h[size_t(k)];
       b->aln_off_h[size_t(k)] = b->aln_bytes;
       b->aln_bytes += 2 * (int64_t(pd.a_len) + pd.b_len);
     }
@@ -1087,9 +1138,11 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     TSQ_TRY(b->cmatrix.ensure(kLetters * kLetters, b->stream, b->async_max));
   }
   TSQ_TRY(b->res_h.ensure(sizeof(ResultDev) * size_t(n)));
-  if (b->out_mode == kOutTrace) {
+  if (b->fill_mode == kOutTrace) {
     TSQ_TRY(b->planes.ensure(size_t(plane_total), b->stream, b->async_max));
     TSQ_TRY(b->plane_off.ensure(sizeof(int64_t) * size_t(n), b->stream, b->async_max));
+  }
+  if (b->out_mode == kOutTrace) {
     TSQ_TRY(b->aln.ensure(size_t(b->aln_bytes), b->stream, b->async_max));
     TSQ_TRY(b->aln_off.ensure(sizeof(int64_t) * size_t(n), b->stream, b->async_max));
     TSQ_TRY(b->aln_h.ensure(size_t(b->aln_bytes)));
@@ -1115,11 +1168,11 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     TSQ_TRY(cudaMemcpyAsync(b->cmatrix.p, sc.cscore, size_t(sc.nclasses) * sc.nclasses, cudaMemcpyHostToDevice,
                             st));
   }
-  if (b->out_mode == kOutTrace && n > 0) {
+  if (b->fill_mode == kOutTrace && n > 0)
     TSQ_TRY(cudaMemcpyAsync(b->plane_off.p, ploff.data(), sizeof(int64_t) * size_t(n), cudaMemcpyHostToDevice, st));
+  if (b->out_mode == kOutTrace && n > 0)
     TSQ_TRY(cudaMemcpyAsync(b->aln_off.p, b->aln_off_h.data(), sizeof(int64_t) * size_t(n), cudaMemcpyHostToDevice,
                             st));
-  }
   if (n > 0) {
     TSQ_TRY(cudaMemcpyAsync(b->shape_g.p, gsel.data(), sizeof(int32_t) * size_t(n), cudaMemcpyHostToDevice, st));
     TSQ_TRY(cudaMemcpyAsync(b->shape_r.p, rsel.data(), sizeof(int32_t) * size_t(n), cudaMemcpyHostToDevice, st));
@@ -1191,7 +1244,7 @@ int enqueue_run(tsq_batch *b) {
   }
   for (int l = 0; l < nl; ++l) {
     const Launch &L = b->launches[size_t(l)];
-    TraceRange lr(fill_range_name(L, b->out_mode));
+    TraceRange lr(fill_range_name(L, b->fill_mode));
     if (L.cta || L.strip) {
       FillArgs a{};
       a.codes = codes_dev(b);
@@ -1215,7 +1268,7 @@ int enqueue_run(tsq_batch *b) {
         a.strip_ctl = b->strip_ws.as<StripCtl>();
         a.strip_rows = reinterpret_cast<uint64_t *>(a.strip_ctl + L.n_pairs);
         a.strip_row_off = b->strip_off.as<int64_t>();
-        TSQ_TRY(launch_strip(L.kind, b->out_mode, b->local, a, L.blocks, b->side));
+        TSQ_TRY(launch_strip(L.kind, b->fill_mode, b->local, a, L.blocks, b->side));
       } else {
         a.bnd = reinterpret_cast<int32_t *>(b->bnd.as<uint8_t>() + L.bnd_offset);
         a.bnd_cols = L.bnd_cols;
@@ -1252,7 +1305,7 @@ int enqueue_run(tsq_batch *b) {
       a.cmatrix = b->cmatrix.as<int8_t>();
       a.nclasses = b->scheme.nclasses;
     }
-    TSQ_TRY(launch_fill(L.R, L.i16, b->out_mode, b->local, a, L.blocks, st));
+    TSQ_TRY(launch_fill(L.R, L.i16, b->fill_mode, b->local, a, L.blocks, st));
   }
   if (forked) {
     TSQ_TRY(cudaEventRecord(b->ev_join, b->side));
@@ -1261,7 +1314,7 @@ int enqueue_run(tsq_batch *b) {
   if (b->n_checked > 0)
     TSQ_TRY(cudaMemcpyAsync(b->rerun_h.p, rerun_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   TSQ_TRY(record(b, 2));
-  if (b->out_mode == kOutTrace) {
+  if (b->fill_mode == kOutTrace) {
     WalkArgs w{};
     w.seqs = seqs_dev(b);
     w.codes = codes_dev(b);
@@ -1273,7 +1326,7 @@ int enqueue_run(tsq_batch *b) {
     w.shape_G = b->shape_g.as<int32_t>();
     w.shape_R = b->shape_r.as<int32_t>();
     w.local = b->local ? 1 : 0;
-    w.emit = 1;
+    w.emit = b->out_mode == kOutTrace ? 1 : 0;
     w.res = b->res.as<ResultDev>();
     w.aln = b->aln.as<char>();
     w.aln_off = b->aln_off.as<int64_t>();

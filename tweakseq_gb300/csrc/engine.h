@@ -143,6 +143,10 @@ struct tsq_batch {
   tsq::Scheme scheme{};
   tsq_params params{};
   int out_mode = tsq::kOutScore;
+  // What the fills compute: out_mode, or traceback planes for identity output
+  // (identity_planes, decided per call: identity_planes_fit).
+  int fill_mode = tsq::kOutScore;
+  bool identity_planes = false, identity_planes_allowed = true;
   bool local = false;
   bool use_graph = false;
   bool autotune = false;
@@ -246,6 +250,8 @@ constexpr int kFillRows = 8;
 int out_mode_of(const tsq_params *p);
 bool lanes16_possible(int out_mode, bool local, int lane);
 bool classes_needed(int out_mode, bool local, int lane);
+// Whether identity output of these pairs runs on traceback planes.
+bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n);
 // TSQ_E_INVALID_ARG for gap costs, mode, output or lane out of range.
 int check_params(const tsq_params *p);
 // TSQ_E_TOO_LARGE for a pair beyond the kernels' value and length ranges.

@@ -177,6 +177,7 @@ int tsq_server::launch(Slot &s, std::vector<std::shared_ptr<Request>> &&reqs, in
   if (!s.batch) {
     s.batch.reset(new tsq_batch());
     s.batch->async_max = SIZE_MAX;  // growth never waits for the other slots
+    s.batch->identity_planes_allowed = false;  // admission counts no planes for identity output
   }
   tsq_params p = s.reqs.front()->params;
   if (p.matrix == TSQ_MATRIX_CUSTOM) {

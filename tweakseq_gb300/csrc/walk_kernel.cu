@@ -286,7 +286,7 @@ __device__ __forceinline__ void walk_one(const WalkArgs &A, int p, uint32_t *s_p
   ResultDev &res = A.res[p];
   WarpSeq<WIN> a{A.seqs + pr.a_off, pr.a_len, s_seq[0], lane}, b{A.seqs + pr.b_off, pr.b_len, s_seq[1], lane};
   const int64_t cap = (int64_t)pr.a_len + pr.b_len;
-  char *out_a = A.aln + A.aln_off[p];
+  char *out_a = A.emit ? A.aln + A.aln_off[p] : nullptr;
   const int G = A.shape_G[p];
   Plane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_plane,
            Plane::band_words(pr.b_len, G), 31 - __clz(G), lane};
