@@ -1300,6 +1300,7 @@ int enqueue_run(tsq_batch *b) {
     a.plane_off = b->plane_off.as<int64_t>();
     a.overflow = b->overflow.as<int32_t>();
     a.max_score = b->scheme.max_score;
+    a.min_score = b->scheme.min_score;
     if (L.i16) {
       a.ccodes = ccodes_dev(b);
       a.cmatrix = b->cmatrix.as<int8_t>();

@@ -20,7 +20,8 @@
 // XO = X - (open + ext) (X clamped at 0 first in local mode) for the next
 // row's F.  F can take X instead of H from the row above because open >= 0
 // makes the F - open - ext candidate redundant, so rows depend on each other
-// through one add-max only.
+// through one add-max only.  (Local score launches have a shorter form: TD
+// below.)
 //
 // Biased halves.  Every value v is held as v + 32768 in an unsigned 16-bit
 // half, compared with the unsigned DPX forms; the proven range keeps every
@@ -210,11 +211,27 @@ __device__ __forceinline__ bool range_has_bad(const uint8_t *p, int len, int t, 
 // warp_rings set (one 32-lane group per warp), the group's rings sit there
 // -- the top ring, then the code ring -- instead of in the block's ring
 // area.
-template <bool LOCAL, bool CHECK, int OUT>
+//
+// TD (local scores without CHECK): the profile's scores carry + (open + ext),
+// so that the diagonal candidate is a plain addition to T = H - (open + ext) of
+// the cell above left, which runs on the FMA pipe; H is not kept, and F comes
+// from T of the row above, with F held at 0 or above, which floors H as well.
+// Per packed cell: the PRMT, three DPX forms and three multiply-adds.
+// TAG: row maxima are taken over units of four steps, from candidates
+// 4 v + 3 - (step mod 4), so that a row's best column costs one and a half ALU
+// instructions per cell and step instead of five; every score of the warp's
+// pairs is below 16,000 and every b below 65,000.  The local score fill was
+// bound by the ALU pipe (92 % busy): 100,000 proteins of median 350 went from
+// 9.11 to 5.77 ms, 20,000 pairs of 320 x 2,000 from 6.43 to 4.32 ms.  (Global
+// scores keep the form above: with TD they gained 1 % on the first and lost 2 %
+// on the second, bound by the chain through the rows rather than by the pipe.)
+template <bool LOCAL, bool CHECK, int OUT, bool TD = false, bool TAG = false>
 __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t *s_mat, uint2 *s_prof,
                                                  uint32_t *s_match, uint8_t *s_rings, int begin, int count,
                                                  int warp_id, int G, int lg, uint8_t *warp_rings = nullptr) {
   static_assert(!(OUT == kOutIdent && LOCAL), "the int16x2 identity fill is global only");
+  static_assert(!TD || (OUT == kOutScore && LOCAL && !CHECK), "local scores only");
+  static_assert(!TAG || TD, "tagged maxima are a part of the TD form");
   using Top = typename Top16<OUT>::T;
   constexpr int R = 8;
   const int P = G * R;   // rows per band
@@ -227,6 +244,8 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
   const uint32_t one = A.one;
   const uint32_t neg_oe2 = 0u - ((uint32_t(oe) << 16) | uint32_t(oe));  // adds -(oe, oe) without borrows
   const uint32_t zero_oe2 = pack2b(-oe, -oe);                          // max(x, 0) - oe floor, local
+  const uint32_t oe2 = 0u - neg_oe2, neg_ge2 = 0u - ((uint32_t(ge) << 16) | uint32_t(ge));
+  (void)oe2, (void)neg_ge2;
   // Opaque constants of the decision arithmetic (multipliers of the FMA
   // pipe's multiply-adds).
   const uint32_t minus_one = 0u - one, k1 = one * 0x00010001u;
@@ -365,11 +384,14 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
       H[r] = pack2b(edge_h(rowA + r + 1, go, ge, LOCAL), edge_h(rowB + r + 1, go, ge, LOCAL));
       T[r] = __viaddmax_u16x2(H[r], noe2, kNeg2);
       E[r] = kNeg2;
-      best[r] = kBias2;
+      best[r] = TAG ? 0x00030003u : kBias2;
       bcol[r] = 0u;
       if constexpr (OUT == kOutIdent) IH[r] = DH[r] = IE[r] = DE[r] = 0u;
     }
     uint32_t hdiag = pack2b(edge_h(rowA, go, ge, LOCAL), edge_h(rowB, go, ge, LOCAL));
+    if constexpr (TD) hdiag = __viaddmax_u16x2(hdiag, noe2, kNeg2);  // TD: the diagonal as T
+    uint32_t cand[R], lead[R];  // TAG: the unit's tagged candidates
+    (void)cand, (void)lead;
     uint32_t outH = kBias2, outF = kNeg2;
     // Identity: counts of the diagonal H and of the bottom row's H and F.
     uint32_t gdI = 0u, gdD = 0u, outIH = 0u, outDH = 0u, outIF = 0u, outDF = 0u;
@@ -495,10 +517,71 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
         // stands for both opened; the decisions subtract from it).
         uint32_t acc1 = 0xCCCCCCCCu, acc2 = 0xCCCCCCCCu;
         uint32_t nz1 = 0u, nz2w = 0u;  // local: rows whose H is above 0
+        // TAG: addend of the step's candidates (4 h - 4 * bias + 3 - k),
+        // the step (of its unit) in both halves, and the update of a row's
+        // best: where the value grew, best takes it (tag 3, so that an equal
+        // value later never beats it) and bcol the step with its last two
+        // bits inverted.
+        const uint32_t tags = (INTERIOR ? uint32_t(3 - k) : uint32_t(3 - (s & 3))) * 0x00010001u - 4u * kBias2;
+        const uint32_t step4 = uint32_t(s & ~3) * 0x00010001u;
+        auto keep_best = [&](int r, uint32_t nb, uint32_t at) {
+          const uint32_t cm = imad(nz2(nb, best[r], minus_one, k1), kffff, 0u);
+          bcol[r] = (bcol[r] & ~cm) | (((nb & 0x00030003u) | at) & cm);
+          best[r] = nb | 0x00030003u;
+        };
+        (void)tags, (void)step4, (void)keep_best;
         // Identity: counts of the cell above (H and F) and of the diagonal.
         uint32_t ciH = upIH, cdH = upDH, ciF = upIF, cdF = upDF;
         uint32_t gI = gdI, gD = gdD;
         (void)acc1, (void)acc2, (void)nz1, (void)nz2w, (void)ciH, (void)cdH, (void)ciF, (void)cdF, (void)gI, (void)gD;
+        // TD: rows in order, F(i+1,j) = max(F(i,j) - ext, T(i,j), 0).
+        auto sweep_td = [&](auto masked_tag, uint32_t keep) {
+          constexpr bool MASKED = decltype(masked_tag)::value;
+          uint32_t f = __vimax3_u16x2(fv, kBias2, kBias2);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const uint32_t sc = score2_dyn(r < 4 ? wa.x : wa.y, r < 4 ? wb.x : wb.y, r);
+            uint32_t e = __viaddmax_u16x2(E[r], nge2, T[r]);
+            const uint32_t h = __vimax3_u16x2(imad(d, one, sc), e, f);
+            uint32_t tn = sub2_imad(h, one, neg_oe2);
+            fv = f;
+            f = __vimax3_u16x2(imad(f, one, neg_ge2), tn, kBias2);
+            if constexpr (TAG) {
+              // The largest candidate of a unit of four steps is its first
+              // maximum, with the step in its last two bits.  (A half out of
+              // range holds anything -- a top row entry past the last column --
+              // and must not carry into the other half: 0 there.)
+              const uint32_t hv = MASKED ? (h & ~keep) | (kBias2 & keep) : h;
+              const uint32_t c = imad(hv, 4u * one, tags);
+              if constexpr (INTERIOR) {
+                if constexpr ((k & 1) == 0)
+                  cand[r] = c;
+                else
+                  lead[r] = __vimax3_u16x2(k == 1 ? best[r] : lead[r], cand[r], c);
+                if constexpr (k == 3) keep_best(r, lead[r], step4);
+              } else {
+                uint32_t nb = __vimax3_u16x2(best[r], c, c);
+                if constexpr (MASKED) nb = (nb & ~keep) | (best[r] & keep);
+                keep_best(r, nb, step4);
+              }
+            } else {
+              // Halves where this cell beats the row's best so far
+              // (strictly, so the first column of a maximum is kept).
+              const uint32_t nb = __vimax3_u16x2(best[r], h, h);
+              uint32_t cm = imad(nz2(nb, best[r], minus_one, k1), kffff, 0u);
+              if constexpr (MASKED) cm &= ~keep;
+              best[r] = (nb & cm) | (best[r] & ~cm);
+              bcol[r] = (bcol[r] & ~cm) | (pack2(jA + 1, jB + 1) & cm);
+            }
+            if constexpr (MASKED) {
+              tn = (tn & ~keep) | (T[r] & keep);
+              e = (e & ~keep) | (E[r] & keep);
+            }
+            d = T[r];
+            T[r] = tn;
+            E[r] = e;
+          }
+        };
         // Rows in order.  Since open >= 0, F(i+1,j) = max(F(i,j) - ext,
         // max(X(i,j) [, 0]) - open - ext) with X = max(D + s, E): the only
         // dependence between rows is one add-max on F.
@@ -608,7 +691,17 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
         // masked sweep alone, whose keep mask is 0 when both halves are in
         // range: their sweeps are large, and fewer copies of them keep the
         // kernel within the instruction cache.)
-        if (INTERIOR || (OUT == kOutScore && vA && vB)) {
+        if constexpr (TD) {
+          if (INTERIOR || (vA && vB)) {
+            hdiag = xo0;
+            sweep_td(BoolTag<false>{}, 0u);
+          } else {
+            // (As below.)
+            const uint32_t keep = (vA ? 0u : 0x0000FFFFu) | (vB ? 0u : 0xFFFF0000u);
+            hdiag = (xo0 & ~keep) | (hdiag & keep);
+            sweep_td(BoolTag<true>{}, keep);
+          }
+        } else if (INTERIOR || (OUT == kOutScore && vA && vB)) {
           hdiag = upH;
           if constexpr (OUT == kOutIdent) {
             gdI = upIH;
@@ -626,7 +719,7 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
           }
           sweep(BoolTag<true>{}, keep);
         }
-        outH = H[R - 1];
+        outH = TD ? imad(T[R - 1], one, oe2) : H[R - 1];
         outF = fv;
         if constexpr (OUT == kOutIdent) {
           outIH = IH[R - 1];
@@ -700,8 +793,12 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const int row = (half ? rowB : rowA) + r;
-            const int32_t v = half ? hi16b(best[r]) : lo16b(best[r]);
-            const int32_t c = half ? int32_t(bcol[r] >> 16) : int32_t(bcol[r] & 0xFFFFu);
+            int32_t v = half ? hi16b(best[r]) : lo16b(best[r]);
+            int32_t c = half ? int32_t(bcol[r] >> 16) : int32_t(bcol[r] & 0xFFFFu);
+            if constexpr (TAG) {  // (the value above its tag; the step, its last two bits inverted)
+              v = int32_t((half ? best[r] >> 16 : best[r] & 0xFFFFu) >> 2);
+              c = (c ^ 3) - t - (half ? G : 0) + 1;
+            }
             if (row < m && v > lbest) {
               lbest = v;
               lrow = row + 1;
@@ -799,7 +896,7 @@ __host__ __device__ constexpr size_t warp_rings16_bytes(int out_mode) {
   return smem16_top_stride(out_mode) + kCodeRing16 + kRingPad;
 }
 
-template <bool LOCAL, bool CHECK, int OUT>
+template <bool LOCAL, bool CHECK, int OUT, bool TD = false>
 __global__ void __launch_bounds__(kThreads16) fill_i16_kernel(const FillArgs A) {
   extern __shared__ __align__(16) uint8_t smem[];
   // Class scores, one 32-byte row per class, then a zero row (index
@@ -810,7 +907,8 @@ __global__ void __launch_bounds__(kThreads16) fill_i16_kernel(const FillArgs A) 
   uint8_t *s_rings = smem + kMatBytes16 + smem16_prof_bytes(A.nclasses) + smem16_match_bytes(OUT, A.nclasses);
   for (int k = threadIdx.x; k < kMatBytes16; k += blockDim.x) {
     const int x = k / kMatRow16, c = k % kMatRow16;
-    s_mat[k] = (x < A.nclasses && c < A.nclasses) ? A.cmatrix[x * A.nclasses + c] : int8_t(0);
+    const int v = (x < A.nclasses && c < A.nclasses) ? A.cmatrix[x * A.nclasses + c] : 0;
+    s_mat[k] = int8_t(TD ? v + A.gap_open + A.gap_extend : v);
   }
   // Code rings start as class 0: a group without a pair still reads its
   // ring, and the step uses what it reads as a profile index unchecked
@@ -831,11 +929,28 @@ __global__ void __launch_bounds__(kThreads16) fill_i16_kernel(const FillArgs A) 
     const int2 w = A.wtasks[idx];
     const int G = w.y >> 16, count = w.y & 0xFFFF;
     const int lg = G == 4 ? 2 : (G == 8 ? 3 : (G == 16 ? 4 : 5));
-    fill16_warp_task<LOCAL, CHECK, OUT>(A, s_mat, s_prof, s_match, s_rings, w.x, count, warp_id, 1 << lg, lg);
+    if constexpr (TD) {
+      // A pair's score is at most max_score times its shorter sequence.
+      const PairDev pr = A.pairs[A.tasks[w.x + min(lane >> lg, count - 1)]];
+      const bool small = int64_t(max(A.max_score, 0)) * (min(pr.a_len, pr.b_len) + 1) < 16000 && pr.b_len < 65000;
+      if (__all_sync(0xffffffffu, small)) {
+        fill16_warp_task<LOCAL, CHECK, OUT, TD, true>(A, s_mat, s_prof, s_match, s_rings, w.x, count, warp_id, 1 << lg,
+                                                      lg);
+        continue;
+      }
+    }
+    fill16_warp_task<LOCAL, CHECK, OUT, TD>(A, s_mat, s_prof, s_match, s_rings, w.x, count, warp_id, 1 << lg, lg);
   }
 }
 
 size_t smem_i16(int out_mode, int nclasses);
+
+// Whether a launch runs the TD form: local scores without CHECK, and every
+// score plus open + ext is a byte from 0 to 127 (BLOSUM62 11/1: 8..23).
+inline bool score16_td(const FillArgs &a, bool local, bool check) {
+  const int64_t oe = int64_t(a.gap_open) + a.gap_extend;
+  return local && !check && a.min_score + oe >= 0 && std::max(a.max_score, 0) + oe <= 127;
+}
 
 // Launch and residency of the int16x2 fill of one output mode (each mode
 // is instantiated in its own translation unit).
@@ -849,6 +964,8 @@ cudaError_t launch_i16(bool check, bool local, const FillArgs &args, int blocks,
       fill_i16_kernel<false, true, OUT><<<blocks, kThreads16, smem, st>>>(a);
     else
       fill_i16_kernel<false, false, OUT><<<blocks, kThreads16, smem, st>>>(a);
+  } else if (OUT == kOutScore && score16_td(a, local, check)) {
+    if constexpr (OUT == kOutScore) fill_i16_kernel<true, false, OUT, true><<<blocks, kThreads16, smem, st>>>(a);
   } else {
     if (check) {
       if (local)
@@ -867,18 +984,23 @@ cudaError_t launch_i16(bool check, bool local, const FillArgs &args, int blocks,
 
 template <int OUT>
 int occupancy_i16(bool check, bool local, size_t smem) {
-  void (*k)(const FillArgs);
+  void (*k)(const FillArgs) = nullptr, (*k2)(const FillArgs) = nullptr;  // (k2: the TD form, of the same residency)
   if constexpr (OUT == kOutIdent) {
     if (local) return 0;
     k = check ? fill_i16_kernel<false, true, OUT> : fill_i16_kernel<false, false, OUT>;
   } else {
     k = check ? (local ? fill_i16_kernel<true, true, OUT> : fill_i16_kernel<false, true, OUT>)
               : (local ? fill_i16_kernel<true, false, OUT> : fill_i16_kernel<false, false, OUT>);
+    if constexpr (OUT == kOutScore)
+      if (local && !check) k2 = fill_i16_kernel<true, false, OUT, true>;
   }
   // The attribute allows the largest profile (26 classes), so that every
   // scheme's launch fits whatever scheme was sized first.
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            int(std::max(smem, smem_i16(OUT, kLetters)))) != cudaSuccess)
+    return 0;
+  if (k2 && cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(std::max(smem, smem_i16(OUT, kLetters)))) != cudaSuccess)
     return 0;
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kThreads16, smem) != cudaSuccess) return 0;

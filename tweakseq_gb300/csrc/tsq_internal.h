@@ -101,6 +101,7 @@ struct FillArgs {
   const int64_t *plane_off;  // byte offset of each pair's planes
   int32_t *overflow;     // int16 CHECK: per pair, 1 when a lane came near 32767
   int32_t max_score;     // largest substitution score of the scheme
+  int32_t min_score;     // smallest
   uint32_t one;          // int16x2 fill: 1, an opaque multiplier for packed subtractions on the IMAD pipe
   const uint8_t *ccodes;  // int16x2 fill: class code per residue (0 for invalid ones), same offsets as codes
   const int8_t *cmatrix;  // int16x2 fill: nclasses x nclasses class scores
