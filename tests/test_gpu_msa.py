@@ -206,3 +206,57 @@ def test_tree_of_more_leaves_than_one_cluster_holds():
     ident, cols = _tied_identities(rng, n, levels=50)
     want = O.guide_tree(O.identity_distances(n, ident, cols), N.TREE["upgma"])
     _same_tree(msa.guide_tree(n, ident, cols, "upgma"), want)
+
+
+# Tiles of 128 columns, warps of 32 rows apart in pairs: ragged columns, rows
+# without a partner, one tile and many, one slice of rows per tile and 152, the
+# even split (110 tiles), and a split that leaves some blocks without rows.
+@pytest.mark.parametrize("nseq,ncols", [(6145, 409), (2500, 1003), (701, 5003), (200, 14000),
+                                        (31, 130001)])
+def test_consensus_pair_counts_at_tile_and_row_edges(nseq, ncols):
+    rng = np.random.default_rng(nseq + ncols)
+    rows = _family_msa(rng, min(nseq, 500), ncols)[rng.integers(0, min(nseq, 500), nseq)]
+    rows[rng.integers(0, nseq, 40), rng.integers(0, ncols, 40)] = rng.integers(0, 256, 40)
+    _check_consensus(rows)
+
+
+def test_consensus_pair_counters_do_not_wrap_and_run_captured():
+    """More rows than 16-bit counters hold per block, all alike; then random
+    rows through the same captured launches."""
+    torch = pytest.importorskip("torch")
+    nseq, ncols = 21_000_003, 4
+    rows = torch.empty((nseq, ncols), dtype=torch.uint8, device="cuda")
+    out = torch.zeros(ncols, dtype=torch.uint8, device="cuda")
+    score = torch.zeros(ncols, dtype=torch.int32, device="cuda")
+    match = torch.zeros(ncols, dtype=torch.int32, device="cuda")
+    nbytes = N.lib().tsq_consensus_scratch_bytes(ncols)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+
+    def run():
+        rc = N.lib().tsq_consensus_device(rows.data_ptr(), nseq, ncols, ncols, -1.0, out.data_ptr(), score.data_ptr(),
+                                          match.data_ptr(), scratch.data_ptr(), nbytes,
+                                          torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+
+    rows[:] = ord("A")
+    rows[:, 2] = ord("-")
+    run()
+    assert out.cpu().numpy().tobytes() == b"AA-A"
+    assert score.tolist() == [4 * (nseq - 1)] * 2 + [nseq - 1] + [4 * (nseq - 1)]
+    assert match.tolist() == [nseq - 1] * 4
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    letters = torch.tensor(list(b"ACDW"), dtype=torch.uint8, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rows.copy_(letters[torch.randint(0, 4, (nseq, ncols), device="cuda", generator=gen)])
+    graph.replay()
+    torch.cuda.synchronize()
+    count = torch.stack([(rows == int(x)).sum(0) for x in letters]).cpu().numpy().astype(np.int64)
+    # A, C, D, W against A, C, D, W (BLOSUM62); a letter's matches are its own
+    # rows, the only positive pairs here.  C's sum is the largest: 0 + 9 - 3 - 2.
+    pair = np.array([[4, 0, -2, -3], [0, 9, -3, -2], [-2, -3, 6, -4], [-3, -2, -4, 11]])
+    sums = pair @ count - np.diag(pair)[:, None]
+    assert (sums.argmax(0) == 1).all()
+    assert np.array_equal(score.cpu().numpy(), sums[1]) and np.array_equal(match.cpu().numpy(), count[1] - 1)
+    assert out.cpu().numpy().tobytes() == bytes(ord("C") if c - 1 >= nseq / 2 else ord("?") for c in count[1])

@@ -26,39 +26,50 @@ namespace {
 
 constexpr int kClasses = 24;  // BLOSUM62 rows 0..22, 23 = gap class
 constexpr int kGapClass = 23;
-constexpr int kBins = 27;  // counted per column: 'A'..'Z', then every other byte
-constexpr int kOtherBin = 26;
+constexpr int kBins = 27;  // counted per column: every byte that is no letter, then 'A'..'Z'
 constexpr int kCountWarps = 8;
 constexpr int kCountThreads = kCountWarps * 32;
 constexpr int kTile = 128;  // columns per block
 
-__constant__ int8_t c_pair[kClasses][kClasses];  // class-vs-class pair scores
-__constant__ uint8_t c_class[256];                // byte -> class
-__constant__ uint8_t c_bin_class[kBins];          // counting bin -> class
+__device__ int8_t c_pair[kClasses][kClasses];  // class-vs-class pair scores
+__device__ uint8_t c_class[256];                  // byte -> class
+__device__ uint8_t c_bin_class[kBins];          // counting bin -> class
 
-// Counting bin of each byte of a word, four at a time: 'A'..'Z' -> 0..25,
-// every other byte -> 26 (per-byte SIMD subtract and compare).
+// Counting bin of each byte of a word, four at a time: 'A'..'Z' -> 1..26,
+// every other byte -> 0.  Six instructions: x = byte - 0x40 modulo the sign, bit
+// 7 of t set where its low seven bits are above 26, bytes with bit 7 in t or x
+// cleared through a sign-replicating permute.
 __device__ __forceinline__ uint32_t bins4(uint32_t v) {
-  const uint32_t d = __vsub4(v, 0x41414141u);
-  const uint32_t lt = __vcmpltu4(d, 0x1a1a1a1au);  // 0xff in the letter bytes
-  return (d & lt) | (0x1a1a1a1au & ~lt);
+  const uint32_t x = v ^ 0x40404040u;
+  const uint32_t t = (x & 0x7F7F7F7Fu) + 0x65656565u;
+  uint32_t mask;
+  asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(mask) : "r"(t | x));
+  return x & ~mask;
 }
 
 // A block covers 128 columns (lane t holds columns t, t+32, t+64, t+96 of
 // the tile, so that its counters fall in bank t) and one slice of the rows,
 // striped over its 8 warps.  With 4-byte-aligned rows a lane reads its 4
 // columns of a row with one 32-bit load, eight rows' loads in flight, bins
-// the four bytes with two SIMD instructions and adds each to its column's
+// the four bytes with six instructions and adds each to its column's
 // bin with one shared-memory atomic -- the one shared-memory operation per
 // byte, which sets the pace.  The counts go to one shared histogram per
 // block, then into the column totals with global atomics.  Only counts: the
 // first row of a class is needed for the winning classes alone and is found
 // afterwards.
+// The three launches of one consensus overlap (programmatic dependent launch):
+// each lets the next start at once, and waits for the one before it to be
+// complete right before it touches what that one wrote.  (With it and the finishing
+// kernel's early reads, 1,000 x 1,000 went from 21 to 16 us.)
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <bool kVec>
 __global__ void __launch_bounds__(kCountThreads) consensus_count_kernel(const uint8_t *__restrict__ rows, int32_t nseq,
                                                                         int32_t ncols, int64_t stride,
                                                                         int32_t rows_per_slice, uint32_t *cnt) {
   __shared__ uint32_t h[kBins][kTile];
+  launch_next();
   for (int k = threadIdx.x; k < kBins * kTile; k += kCountThreads) (&h[0][0])[k] = 0u;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -101,6 +112,7 @@ __global__ void __launch_bounds__(kCountThreads) consensus_count_kernel(const ui
       }
     }
   }
+  wait_previous();
   __syncthreads();
   for (int e = threadIdx.x; e < kBins * kTile; e += kCountThreads) {
     const int bin = e / kTile, slot = e % kTile;
@@ -111,7 +123,136 @@ __global__ void __launch_bounds__(kCountThreads) consensus_count_kernel(const ui
   }
 }
 
+// Pair counting, for all but small alignments.  The kernel above issues one
+// shared-memory atomic per byte; here one atomic counts two rows' bytes of a
+// column: a block, alone on its SM, holds 128 columns' counts of the 27 x 27
+// bin pairs in 16 bits (182 KB; two columns' counters share a word, at
+// (u / 2) * 32 + lane, so a warp's atomics fall in 32 banks), and folds them
+// into the column totals when it leaves a tile.  The address is one two-term
+// dot product of the pair's bins.  A warp loads its next 8 rows while it counts
+// 8.  All blocks of a row range run at the same time, so that the sectors that
+// two tiles share come from L2 once read.  It waits on its loads (with 16 rows
+// at once and none ahead 2 us more).
+// All launches of one call, before and after: 100,003 x 2,000 84 -> 61 us (200 MB,
+// 4.5 TB/s while counting; a plain copy reads and writes 6.8), 50,000 x 1,000
+// 63 -> 28, 10,000 x 1,000 58 -> 22.  Zeroing and folding cost about 5 us, so
+// below kPairBytes the kernel above is the better one: 2,000 x 1,000 21.0 and
+// 20.9 us, 1,000 x 1,000 15.9 and 22.3.
+constexpr int kPairWarps = 32;
+constexpr int kPairThreads = kPairWarps * 32;
+constexpr int kPairRows = 8;               // rows per warp and iteration
+constexpr int kPairUnit = 2 * kPairWarps;  // rows: the grain of the blocks' shares
+constexpr int kPairWords = kTile / 2;                  // counter words per bin pair
+constexpr size_t kPairSmem = size_t(kBins) * kBins * kPairWords * 4;
+constexpr int64_t kPairBytes = 2500000;  // alignments from this size on
+constexpr int64_t kPairMaxUnits = 65535 / (kPairUnit / 2);  // per fold: a counter counts at most 65,535 pairs
+
+__global__ void __launch_bounds__(kPairThreads, 1)
+    consensus_pairs_kernel(const uint8_t *__restrict__ rows, int32_t nseq, int32_t ncols, int64_t stride,
+                           int64_t units_per_tile, int32_t tiles, int32_t slices, uint32_t *cnt) {
+  extern __shared__ __align__(16) uint32_t pairs[];
+  launch_next();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // slices > 0: one tile, one of `slices` shares of its rows; 0: an even share
+  // of the rows of all tiles, one after the other.
+  const int64_t units = slices ? units_per_tile : units_per_tile * tiles;
+  const int32_t part = slices ? int32_t(blockIdx.x) / tiles : int32_t(blockIdx.x), parts = slices ? slices : gridDim.x;
+  const int64_t u0 = slices ? units_per_tile * (int32_t(blockIdx.x) % tiles) : 0;
+  int64_t u = u0 + units * part / parts;
+  const int64_t u_end = u0 + units * (part + 1) / parts;
+  const uint32_t base = uint32_t(__cvta_generic_to_shared(pairs)) + 4u * lane;
+  constexpr uint32_t kRow = kPairWords * 4;                      // bytes per bin pair
+  constexpr uint32_t kWeights = (kRow << 16) | (kBins * kRow);   // second bin, first bin
+  static_assert(kBins * kRow < 65536, "weights of 16 bits");
+  auto inc = [](uint32_t addr, uint32_t v) { asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); };
+  while (u < u_end) {
+    const int64_t tile = u / units_per_tile;
+    const int64_t stop = min(min(u_end, (tile + 1) * units_per_tile), u + kPairMaxUnits);
+    const int64_t row0 = (u - tile * units_per_tile) * kPairUnit;
+    const int64_t row1 = min(int64_t(nseq), (stop - tile * units_per_tile) * kPairUnit);
+    const int32_t c0 = int32_t(tile) * kTile;
+    for (int k = threadIdx.x; k < int(kPairSmem / 16); k += kPairThreads)
+      reinterpret_cast<uint4 *>(pairs)[k] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    const int32_t mc = c0 + 4 * lane;
+    const int nvalid = max(0, min(4, ncols - mc));
+    const uint8_t *p = rows + mc;
+    auto load = [&](int64_t r) -> uint32_t {  // (ragged last columns: bytes)
+      uint32_t v = 0;
+      for (int k = 0; k < nvalid; ++k) v |= uint32_t(__ldg(p + r * stride + k)) << (8 * k);
+      return v;
+    };
+    // Two rows' bytes of the lane's four columns (columns past the last one
+    // count what is never read).
+    auto count = [&](uint32_t va, uint32_t vb) {
+      const uint32_t a = bins4(va), b = bins4(vb);
+      const uint32_t lo = __byte_perm(a, b, 0x5140u), hi = __byte_perm(a, b, 0x7362u);
+      inc(__dp2a_lo(kWeights, lo, base), 1u);
+      inc(__dp2a_hi(kWeights, lo, base), 0x10000u);
+      inc(__dp2a_lo(kWeights, hi, base) + 128u, 1u);
+      inc(__dp2a_hi(kWeights, hi, base) + 128u, 0x10000u);
+    };
+    if (nvalid > 0) {
+      int64_t r = row0 + w;
+      if (nvalid == 4) {
+        const int64_t step = int64_t(kPairWarps) * stride;
+        const uint8_t *q0 = p + r * stride;
+        // (The next rows are loaded before these are counted.)
+        uint32_t v[kPairRows], next[kPairRows];
+        auto fetch = [&](uint32_t *to) {
+          const uint8_t *qq = q0;
+#pragma unroll
+          for (int q = 0; q < kPairRows; ++q, qq += step) to[q] = __ldg(reinterpret_cast<const uint32_t *>(qq));
+          q0 = qq;
+          r += kPairRows * kPairWarps;
+        };
+        auto full = [&]() { return r + (kPairRows - 1) * kPairWarps < row1; };
+        if (full()) {
+          fetch(v);
+          while (full()) {
+            fetch(next);
+#pragma unroll
+            for (int q = 0; q < kPairRows; q += 2) count(v[q], v[q + 1]);
+#pragma unroll
+            for (int q = 0; q < kPairRows; ++q) v[q] = next[q];
+          }
+#pragma unroll
+          for (int q = 0; q < kPairRows; q += 2) count(v[q], v[q + 1]);
+        }
+        for (; r + kPairWarps < row1; r += 2 * kPairWarps, q0 += 2 * step)
+          count(__ldg(reinterpret_cast<const uint32_t *>(q0)), __ldg(reinterpret_cast<const uint32_t *>(q0 + step)));
+      } else {
+        for (; r + kPairWarps < row1; r += 2 * kPairWarps) count(load(r), load(r + kPairWarps));
+      }
+      wait_previous();
+      if (r < row1) {  // a row without a partner
+        const uint32_t b = bins4(load(r));
+        for (int k = 0; k < nvalid; ++k) atomicAdd(&cnt[int64_t(mc + k) * kBins + ((b >> (8 * k)) & 0xffu)], 1u);
+      }
+    }
+    wait_previous();
+    __syncthreads();
+    // Fold: a bin's count is its row's and its column's sum of the table.
+    for (int e = threadIdx.x; e < kBins * kPairWords; e += kPairThreads) {
+      const int bin = e / kPairWords, slot = e % kPairWords;
+      uint32_t s0 = 0u, s1 = 0u;
+#pragma unroll 9
+      for (int y = 0; y < kBins; ++y) {
+        const uint32_t x = pairs[(bin * kBins + y) * kPairWords + slot], z = pairs[(y * kBins + bin) * kPairWords + slot];
+        s0 += (x & 0xffffu) + (z & 0xffffu);
+        s1 += (x >> 16) + (z >> 16);
+      }
+      const int32_t col = c0 + 4 * (slot & 31) + 2 * (slot >> 5);
+      if (s0 != 0u && col < ncols) atomicAdd(&cnt[int64_t(col) * kBins + bin], s0);
+      if (s1 != 0u && col + 1 < ncols) atomicAdd(&cnt[int64_t(col + 1) * kBins + bin], s1);
+    }
+    __syncthreads();
+    u = stop;
+  }
+}
+
 __global__ void consensus_init_kernel(uint32_t *cnt, int64_t n) {
+  launch_next();
   for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x)
     cnt[k] = 0u;
 }
@@ -125,7 +266,7 @@ __global__ void consensus_init_kernel(uint32_t *cnt, int64_t n) {
 constexpr int kFinishWarps = 8;
 __global__ void __launch_bounds__(kFinishWarps * 32)
     consensus_finish_kernel(const uint8_t *__restrict__ rows, int32_t nseq, int32_t ncols, int64_t stride,
-                            double plurality, const uint32_t *__restrict__ cnt, uint8_t *out, int32_t *best_score,
+                            double plurality, const uint32_t *cnt, uint8_t *out, int32_t *best_score,
                             int32_t *best_matches) {
   __shared__ uint8_t cls[256];
   __shared__ int8_t pair[kClasses][kClasses + 1];
@@ -136,13 +277,16 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int32_t col = blockIdx.x * kFinishWarps + w;
   __shared__ uint32_t bin_s[kFinishWarps][kBins];
-  if (col < ncols && lane < kBins) bin_s[w][lane] = cnt[int64_t(col) * kBins + lane];
+  // The first 32 rows' bytes of the column: usually all the scan below reads.
+  const int first_byte = col < ncols && lane < nseq ? int(rows[int64_t(lane) * stride + col]) : 0;
+  const int bin_class = lane < kBins ? int(c_bin_class[lane]) : -1;
+  wait_previous();
+  if (col < ncols && lane < kBins) bin_s[w][lane] = __ldcg(cnt + int64_t(col) * kBins + lane);
   __syncwarp();
-  if (col < ncols && lane < kClasses) {  // fold the bins into the classes
-    uint32_t c = 0u;
-    for (int b = 0; b < kBins; ++b) c += c_bin_class[b] == lane ? bin_s[w][b] : 0u;
-    n_s[w][lane] = c;
-  }
+  // Fold the bins into the classes: each lane collects the bins of its class.
+  uint32_t mine = 0u;
+  for (int b = 0; b < kBins; ++b) mine += __shfl_sync(0xffffffffu, bin_class, b) == lane ? bin_s[w][b] : 0u;
+  if (lane < kClasses) n_s[w][lane] = mine;
   __syncthreads();
   if (col >= ncols) return;
   const int x = lane < kClasses ? lane : 0;
@@ -166,25 +310,28 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   }
   const uint32_t winners = __ballot_sync(0xffffffffu, present && sx == bs);  // classes holding the best sum
   int32_t r = -1;
-  int c = 0;
+  int c = 0, shown = 0;
   for (int32_t r0 = 0; r0 < nseq; r0 += 32) {
     const int32_t rr = r0 + lane;
-    const int cl = rr < nseq ? int(cls[rows[int64_t(rr) * stride + col]]) : 0;
+    const int byte = r0 == 0 ? first_byte : rr < nseq ? int(rows[int64_t(rr) * stride + col]) : 0;
+    const int cl = int(cls[byte]);
     const uint32_t hit = __ballot_sync(0xffffffffu, rr < nseq && ((winners >> cl) & 1u));
     if (hit) {
       const int first = __ffs(hit) - 1;
       r = r0 + first;
       c = __shfl_sync(0xffffffffu, cl, first);
+      shown = __shfl_sync(0xffffffffu, byte, first);
       break;
     }
   }
   if (r < 0) {  // (a winning class always occurs; stays in bounds regardless)
     r = nseq - 1;
-    c = cls[rows[int64_t(r) * stride + col]];
+    shown = rows[int64_t(r) * stride + col];
+    c = cls[shown];
   }
   const int64_t bm = __shfl_sync(0xffffffffu, mt, c);
   if (lane == 0) {
-    out[col] = double(bm) >= plurality ? rows[int64_t(r) * stride + col] : uint8_t('?');
+    out[col] = double(bm) >= plurality ? uint8_t(shown) : uint8_t('?');
     if (best_score) best_score[col] = int32_t(bs);
     if (best_matches) best_matches[col] = int32_t(bm);
   }
@@ -198,8 +345,8 @@ void class_tables(int8_t pair[kClasses][kClasses], uint8_t cls[256], uint8_t bin
   for (int b = 0; b < 256; ++b) cls[b] = kGapClass;
   for (int k = 0; k < 23; ++k) cls[uint8_t(kOrder[k])] = uint8_t(k);
   cls[uint8_t('J')] = cls[uint8_t('O')] = cls[uint8_t('U')] = 22;
-  for (int b = 0; b < 26; ++b) bin_class[b] = cls[uint8_t('A' + b)];
-  bin_class[kOtherBin] = kGapClass;
+  bin_class[0] = kGapClass;
+  for (int b = 0; b < 26; ++b) bin_class[1 + b] = cls[uint8_t('A' + b)];
   for (int x = 0; x < kClasses; ++x)
     for (int y = 0; y < kClasses; ++y) {
       if (x == kGapClass && y == kGapClass)
@@ -223,6 +370,8 @@ cudaError_t upload_tables() {
   e = cudaMemcpyToSymbol(c_pair, pair, sizeof(pair));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_class, cls, sizeof(cls));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_bin_class, bin_class, sizeof(bin_class));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(consensus_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem));
   if (e == cudaSuccess) done_dev = dev;
   return e;
 }
@@ -248,6 +397,20 @@ cudaError_t consensus_enqueue(const uint8_t *d_rows, int32_t nseq, int32_t ncols
   uint32_t *cnt = static_cast<uint32_t *>(scratch);
   const int64_t entries = int64_t(ncols) * kBins;
   consensus_init_kernel<<<int(std::min<int64_t>((entries + 255) / 256, 4096)), 256, 0, stream>>>(cnt, entries);
+  // The next two launches may start before the one ahead of them ends.
+  cudaLaunchAttribute early[1] = {};
+  early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early[0].val.programmaticStreamSerializationAllowed = 1;
+  auto launch = [&](auto kernel, dim3 grid, int threads, size_t smem, auto... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+  };
   // Enough blocks for every SM several times over: split the rows into
   // slices when the columns alone do not give them.
   const int32_t col_tiles = (ncols + kTile - 1) / kTile;
@@ -257,15 +420,22 @@ cudaError_t consensus_enqueue(const uint8_t *d_rows, int32_t nseq, int32_t ncols
   per = std::max(per, 8 * kCountWarps);
   slices = (nseq + per - 1) / per;
   const bool vec = stride % 4 == 0 && reinterpret_cast<uintptr_t>(d_rows) % 4 == 0;
-  if (vec)
-    consensus_count_kernel<true><<<dim3(col_tiles, slices), kCountThreads, 0, stream>>>(d_rows, nseq, ncols, stride,
-                                                                                      per, cnt);
-  else
-    consensus_count_kernel<false><<<dim3(col_tiles, slices), kCountThreads, 0, stream>>>(d_rows, nseq, ncols, stride,
-                                                                                       per, cnt);
-  consensus_finish_kernel<<<(ncols + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, stream>>>(
-      d_rows, nseq, ncols, stride, plurality, cnt, d_out, d_score, d_matches);
-  return cudaGetLastError();
+  if (vec && int64_t(nseq) * ncols >= kPairBytes) {
+    const int64_t upt = (int64_t(nseq) + kPairUnit - 1) / kPairUnit;
+    const int sms = sm_count();
+    // As many slices as give every SM a block; an even split where that
+    // would leave more than 15 % of them idle.
+    int32_t ps = sms / col_tiles;
+    if (int64_t(ps) * col_tiles * 100 < int64_t(sms) * 85) ps = 0;
+    e = launch(consensus_pairs_kernel, dim3(ps ? ps * col_tiles : sms), kPairThreads, kPairSmem, d_rows, nseq, ncols,
+               stride, upt, col_tiles, ps, cnt);
+  } else {
+    e = launch(vec ? consensus_count_kernel<true> : consensus_count_kernel<false>, dim3(col_tiles, slices),
+               kCountThreads, 0, d_rows, nseq, ncols, stride, per, cnt);
+  }
+  if (e != cudaSuccess) return e;
+  return launch(consensus_finish_kernel, dim3((ncols + kFinishWarps - 1) / kFinishWarps), kFinishWarps * 32, 0, d_rows,
+                nseq, ncols, stride, plurality, static_cast<const uint32_t *>(cnt), d_out, d_score, d_matches);
 }
 
 struct ConsensusCache {
