@@ -89,7 +89,9 @@ typedef struct {
  * is aligned against b[b_begin:b_end].  Fields a mode does not compute are
  * -1 (begins for TSQ_OUT_SCORE local; n_ident/n_cols for TSQ_OUT_SCORE).
  * aln_a / aln_b are NUL-terminated, allocated by the library for
- * TSQ_OUT_ALIGNMENT and released by tsq_result_free; otherwise NULL. */
+ * TSQ_OUT_ALIGNMENT and released by tsq_result_free; otherwise NULL.  The rows
+ * of pairs of one call may share blocks of memory of up to 256 KB, each freed
+ * with the last result that uses it. */
 typedef struct {
   int32_t score;
   int32_t a_begin, a_end, b_begin, b_end;

@@ -102,35 +102,37 @@ def _per_pair_status(rc: int, raw: np.ndarray) -> bool:
     return rc in (N.E_INVALID_RESIDUE, N.E_TIMEOUT, N.E_TOO_LARGE) and bool((raw["status"] == rc).any())
 
 
+_TABLE_DTYPE = np.dtype([(k, np.int32) for k in
+                         ("score", "a_begin", "a_end", "b_begin", "b_end", "n_ident", "n_cols", "status")])
+
+
 def _collect(raw: np.ndarray, strings: bool) -> BatchResult:
     L = N.lib()
-    table = np.empty(len(raw), dtype=[(k, np.int32) for k in
-                                      ("score", "a_begin", "a_end", "b_begin", "b_end", "n_ident", "n_cols",
-                                       "status")])
-    for k in table.dtype.names:
-        table[k] = raw[k]
+    # The table's columns are the first eight words of a result.
+    table = np.empty(len(raw), dtype=_TABLE_DTYPE)
+    words = len(_TABLE_DTYPE)
+    table.view(np.int32).reshape(len(raw), words)[:] = raw.view(np.int32).reshape(
+        len(raw), raw.itemsize // 4)[:, :words]
     sa = sb = None
     if strings:
         # All strings in one copy (tsq_results_strings), then slices of one
         # decoded text: a string_at per string costs more than the alignment.
         ptr = raw.ctypes.data if len(raw) else None
-        total = L.tsq_results_strings(ptr, len(raw), None, 0)
-        N.check(min(total, 0), "tsq_results_strings")
-        buf = np.empty(max(total, 1), dtype=np.uint8)
-        got = L.tsq_results_strings(ptr, len(raw), buf.ctypes.data, total)
-        N.check(min(got, 0), "tsq_results_strings")
-        text = buf[:total].tobytes().decode("ascii")
-        has = ((raw["aln_a"] != 0) & (raw["aln_b"] != 0)).tolist()
+        has = (raw["aln_a"] != 0) & (raw["aln_b"] != 0)
         lens = np.where(has, raw["n_cols"], 0).astype(np.int64)
-        ends = np.cumsum(2 * lens).tolist()
-        sa, sb = [], []
-        for h, c, e in zip(has, lens.tolist(), ends):
-            if h:
-                sa.append(text[e - 2 * c:e - c])
-                sb.append(text[e - c:e])
-            else:
-                sa.append(None)
-                sb.append(None)
+        room = 2 * int(np.maximum(lens, 0).sum())
+        buf = np.empty(max(room, 1), dtype=np.uint8)
+        got = L.tsq_results_strings(ptr, len(raw), buf.ctypes.data, room)
+        N.check(min(got, 0), "tsq_results_strings")
+        text = str(memoryview(buf)[:room], "ascii")
+        ends = np.cumsum(2 * lens)
+        mids = (ends - lens).tolist()
+        begins = (ends - 2 * lens).tolist()
+        ends = ends.tolist()
+        sa = [text[i:j] for i, j in zip(begins, mids)]
+        sb = [text[i:j] for i, j in zip(mids, ends)]
+        for k in np.flatnonzero(~has).tolist():
+            sa[k] = sb[k] = None
         L.tsq_results_free(raw.ctypes.data, len(raw))
     return BatchResult(table, sa, sb)
 

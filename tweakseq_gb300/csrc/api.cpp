@@ -257,15 +257,11 @@ int tsq_version(int32_t *abi_version, const char **build) {
 }
 
 void tsq_result_free(tsq_result *r) {
-  if (!r) return;
-  std::free(r->aln_a);
-  std::free(r->aln_b);
-  r->aln_a = r->aln_b = nullptr;
+  if (r) tsq::free_rows(r, 1);
 }
 
 void tsq_results_free(tsq_result *r, int64_t n) {
-  if (!r) return;
-  for (int64_t k = 0; k < n; ++k) tsq_result_free(&r[k]);
+  if (r) tsq::free_rows(r, n);
 }
 
 int64_t tsq_results_strings(const tsq_result *r, int64_t n, char *buf, int64_t buf_len) {

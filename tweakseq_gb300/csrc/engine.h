@@ -267,6 +267,8 @@ Range16 range16(const tsq_params *p, const Scheme &sc, int32_t a_len, int32_t b_
 // status is OK), its two rows from the walker's output of 2 * cap bytes.
 // Returns TSQ_OK, or TSQ_E_CUDA / TSQ_E_NOMEM when the rows cannot be taken.
 int collect_one(const ResultDev &d, const char *rows, int64_t cap, tsq_result &o);
+// Releases the rows of results that collect_one filled (those without are left).
+void free_rows(tsq_result *r, int64_t n);
 
 // The plain form's one-pair path (pair.cpp).  One object per host thread.
 struct PairPath {
