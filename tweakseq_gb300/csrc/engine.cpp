@@ -732,6 +732,10 @@ int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts
 // warp is as fast as strips up to about 600 steps (20 pairs x 150: 0.067 ms
 // either way).  Identity output's long form is a CTA of 8 warps, worth its
 // int32 cells from 20,000 steps.
+// Pairs of a strip launch up to which each is walked by a block's warps: 20 pairs
+// x 3,000 0.17 -> 0.05 ms, 300 x 3,000 0.20 -> 0.09, 300 x 1,200 0.10 -> 0.07; with
+// more, a warp for each pair fills the GPU and walks no cell twice.
+constexpr int32_t kManyWalks = 1024;
 constexpr double kLongSteps = 600.0, kLongShare = 1.5, kLongStepsCta = 20000.0;
 
 // The strip launch of the pairs at [s, e) of the sorted order: its units,
@@ -764,7 +768,11 @@ void plan_strips(tsq_batch *b, PlanScratch &ps, int64_t s, int64_t e, StripKind 
       list.push_back(make_int2(int32_t(q - s), st));
     }
     off.push_back(entries);
-    entries += strips > 1 ? (int64_t(pd.b_len) + 15) & ~int64_t(15) : 0;
+    // The hand-over row; later the walk's records where those need the room.
+    int64_t room = strips > 1 ? pd.b_len : 0;
+    if (b->fill_mode == kOutTrace && pd.a_len >= kWalkRecRows) room = std::max<int64_t>(room, (pd.a_len + 2) / 2);
+    entries += (room + 15) & ~int64_t(15);
+    L.max_rows = std::max(L.max_rows, pd.a_len);
   }
   for (SortRec &r : key) r.key = most - r.key;
   radix_sort(key, ps.tmp, bit_width(most));
@@ -1402,7 +1410,29 @@ int enqueue_run(tsq_batch *b) {
     w.aln = b->aln.as<char>();
     w.aln_off = b->aln_off.as<int64_t>();
     TraceRange wr("walk");
-    TSQ_TRY(launch_walk(w, st));
+    // Pairs of a strip launch by one block each, beside the others, as long as
+    // a warp for each pair would leave the GPU idle.
+    for (const Launch &L : b->launches) {
+      if (!L.strip || L.n_pairs > kManyWalks) continue;
+      w.skip_begin = L.task_begin;
+      w.skip_end = L.task_begin + L.n_pairs;
+      WalkArgs s = w;
+      s.tasks += L.task_begin;
+      s.n_tasks = L.n_pairs;
+      s.rec_rows = reinterpret_cast<uint64_t *>(b->strip_ws.as<StripCtl>() + L.n_pairs);
+      s.rec_off = b->strip_off.as<int64_t>();
+      const bool beside = L.n_pairs < w.n_tasks;
+      if (beside) {
+        TSQ_TRY(cudaEventRecord(b->ev_fork, st));
+        TSQ_TRY(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
+      }
+      TSQ_TRY(launch_walk_block(s, L.R, L.max_rows, beside ? b->side : st));
+      if (beside) TSQ_TRY(cudaEventRecord(b->ev_join, b->side));
+    }
+    if (w.skip_end - w.skip_begin < w.n_tasks) {
+      TSQ_TRY(launch_walk(w, st));
+      if (w.skip_end > w.skip_begin) TSQ_TRY(cudaStreamWaitEvent(st, b->ev_join, 0));
+    }
   }
   TSQ_TRY(record(b, 3));
   return TSQ_OK;

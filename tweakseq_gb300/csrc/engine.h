@@ -58,7 +58,7 @@ struct Launch {
   bool strip = false;  // long pairs in strips (fill_strip.cu); pairs tasks[task_begin, +n_pairs), units
                        // [wt_begin, +n_wtasks) of the warp-task list
   StripKind kind = kStrip32;
-  int32_t n_pairs = 0;
+  int32_t n_pairs = 0, max_rows = 0;
   int32_t task_begin = 0;
   int32_t wt_begin = 0, n_wtasks = 0;  // slice of the warp-task list
   int32_t blocks = 0;

@@ -126,7 +126,9 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   const int64_t off_res = off_ccodes + align256(len + kPad);
   const int64_t down_bytes = int64_t(sizeof(ResultDev)) + (emit ? 2 * len : 0);  // record, then a and b rows
   const int64_t off_bnd = off_res + align256(down_bytes);
-  const int64_t bnd_bytes = n_units > 1 ? (int64_t(lb) + 15) / 16 * 16 * 8 : 0;  // the strips' hand-over row
+  // The strips' hand-over row, later the walk's records where those need it.
+  int64_t bnd_bytes = n_units > 1 ? (int64_t(lb) + 15) / 16 * 16 * 8 : 0;
+  if (out_mode != kOutScore && la >= kWalkRecRows) bnd_bytes = std::max(bnd_bytes, (int64_t(la) + 2) / 2 * 8);
   const int64_t off_planes = off_bnd + align256(bnd_bytes);
   const int64_t plane_total = walk ? plane_bytes(la, lb, shp) : 0;
   const int64_t dev_bytes = off_planes + std::max<int64_t>(plane_total, 16);
@@ -207,7 +209,9 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
     w.res = res;
     w.aln = rows;
     w.aln_off = reinterpret_cast<const int64_t *>(d + kOffAlnOff);
-    PAIR_TRY(launch_walk(w, st));
+    w.rec_rows = fa.strip_rows;
+    w.rec_off = fa.strip_row_off;
+    PAIR_TRY(launch_walk_block(w, shp.R, la, st));
   }
   PAIR_TRY(cudaMemcpyAsync(pp->down.p, res, size_t(down_bytes), cudaMemcpyDeviceToHost, st));
   PAIR_TRY(cudaStreamSynchronize(st));

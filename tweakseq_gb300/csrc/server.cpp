@@ -441,7 +441,7 @@ int tsq_server_submit(tsq_server *s, const uint8_t *seqs, int64_t seqs_len, cons
         return TSQ_E_INVALID_ARG;
       r->cells += int64_t(d.a_len) * d.b_len;
       r->max_n = std::max(r->max_n, d.b_len);
-      bytes += 8 * int64_t(d.b_len) + 40;  // a long pair's hand-over row and record
+      bytes += 8 * std::max<int64_t>(d.b_len, d.a_len / 2) + 64;  // a long pair's hand-over row (or walk records) and record
       if (p->output == TSQ_OUT_ALIGNMENT)
         bytes += tsq::plane_bytes(d.a_len, d.b_len, tsq::Shape{32, 8, 0}) + 2 * (int64_t(d.a_len) + d.b_len);
     }

@@ -136,6 +136,12 @@ struct WalkArgs {
   ResultDev *res;
   char *aln;                 // per pair: 2 * cap bytes (a row then b row)
   const int64_t *aln_off;
+  int32_t skip_begin, skip_end;  // launch_walk: tasks that another launch walks
+  // launch_walk_block: per task, (a_len + 2) / 2 entries for the path's records
+  // (used by pairs whose records do not fit shared memory).
+  uint64_t *rec_rows;
+  const int64_t *rec_off;
+  int32_t rec_words;
 };
 
 // Host-side helpers (scheme.cpp).
@@ -188,6 +194,12 @@ struct StripLoad {
   StripKind pick(int out_mode, int sms, bool allow16) const;
 };
 cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st);
+// The pairs of a strip launch, one block each; max_rows: their longest a.
+// Pairs of at least kWalkRecRows rows need room for their records.
+constexpr int32_t kWalkRecRows = 32768;
+cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st);
+// The pairs of a strip launch, one block each; max_rows: their longest a.
+cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st);
 // Residues -> letter codes and, when clut_dev / ccodes are set, score
 // classes.
 cudaError_t launch_encode(const uint8_t *seqs, int64_t len, const uint8_t *lut_dev, uint8_t *codes,

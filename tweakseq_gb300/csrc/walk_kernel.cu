@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kWarpWalkWarps * 32) walk_warp_kernel(const Wa
   __shared__ uint8_t s_seq[kWarpWalkWarps][2][WIN];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * kWarpWalkWarps + w;
-  if (k >= A.n_tasks) return;
+  if (k >= A.n_tasks || (k >= A.skip_begin && k < A.skip_end)) return;
   const int p = A.tasks[k];
   if (A.res[p].status != TSQ_OK) return;
   const int R = A.shape_R[p];
@@ -322,6 +322,282 @@ __global__ void __launch_bounds__(kWarpWalkWarps * 32) walk_warp_kernel(const Wa
     else
       walk_one<8, 32, 4, WIN>(A, p, s_plane[w], s_seq[w], lane);
   }
+}
+
+// ---- one pair by many warps ---------------------------------------------
+//
+// A walk is a chain of dependent steps, about 50 ns a column on an idle GPU.
+// For the pairs of the strip fill, few and long, the rows are cut into
+// segments, one per warp of a block.  All warps walk their segment at once: the
+// lowest from the true end cell, the others from a guessed cell of their
+// lowest row (on the line from the end cell to the start).  Traceback paths that
+// start near each other meet after a few cells and are one from there on, so
+// what a warp walked is the true path but for its beginning.  Then every
+// segment whose true entry -- the cell and state where the path of the segment
+// below leaves it -- is not the one it started from walks again from there, until it
+// meets what it recorded; rounds go on until every segment's entry is what
+// the one below hands it.  The lowest segment is exact at once, and each round
+// makes at least one more so: at most as many rounds as segments, the time of
+// the plain walk, whatever the guesses; two or three where the sequences are
+// related.  Every cell is a cell of the true path in the end, whichever way.
+//
+// A row's record: the column and state in which the path arrives in it, and
+// how it leaves (diagonal, up, or not at all): its columns follow from that
+// and the next row's arrival, so the gapped rows are written afterwards by all
+// warps at offsets from a sum over them.
+// One 20 kb pair (DNA, 10 % substitutions, 2 % indels) 1.10 -> 0.10 ms, 23 pairs of
+// 10 to 50 kb 2.60 -> 0.33 ms, one protein pair of 383 residues 20 -> 12 us.  What is
+// left is the longest segment's own chain of steps.
+constexpr uint32_t kRecCol = 0xFFFFFu;  // column (pairs are below 2^20), state << 20, leave << 22
+constexpr uint32_t kRecArrival = 0x3FFFFFu;
+constexpr uint32_t kLeaveDiag = 0u << 22, kLeaveUp = 1u << 22, kLeaveStop = 2u << 22;
+constexpr uint32_t kExitStop = 1u << 30, kExitBad = 1u << 31;  // exits: the path ends inside; the planes make no sense
+constexpr int kSegRows = 64;  // fewest rows of a segment: paths meet within some tens of rows
+constexpr int kWinSteps4 = 32, kWinLanes4 = 14, kWinSteps8 = 64, kWinLanes8 = 9, kWinWords = 576;
+constexpr int kMaxSegs = 32;
+static_assert(kWalkRecRows < ((222 << 10) / 4 - kMaxSegs * kWinWords), "shorter pairs' records fit");
+constexpr size_t kWalkSmem = size_t(222) << 10;  // dynamic shared memory of a block, at most
+
+struct SegWalk {
+  uint32_t exit;  // arrival in row `lo`, or kExitStop and the column where the path ends
+  int floor;      // last row walked
+  bool met;       // met the recorded path: exit and floor are those it had
+};
+
+// Walks rows i = hi .. lo + 1 from (hi, j, state); writes their records.
+// floor: the last row of the path recorded before (hi + 1: none).
+template <class Plane>
+__device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi, int lo, int j, int state, bool local,
+                                                int floor, int lane) {
+  int i = hi;
+  uint32_t arrival = uint32_t(j) | uint32_t(state) << 20;
+  pl.set_row(i);
+  for (;;) {
+    if (state == 0) {
+      if (j == 0) {
+        if (local) {
+          if (lane == 0) rec[i] = arrival | kLeaveStop;
+          return {kExitStop, i, false};
+        }
+        // Global, left column: up to row 0.
+        for (int k = i - lane; k > lo; k -= 32) rec[k] = (k == i ? arrival : 0u) | kLeaveUp;
+        return {0u, lo + 1, false};
+      }
+      const int hd = pl.nib(j) & 3;
+      if (hd == kDirDiag) {
+        // A run of diagonal moves at once: lane k leaves row i - k.
+        const uint32_t dm = pl.diag_mask(i, j);
+        const int p = min(dm == 0xffffffffu ? 32 : __ffs(~dm) - 1, i - lo);
+        // Arrivals of rows i - 1 - lane, the run's and the one it leads to.
+        const bool same = lane < p && i - 1 - lane >= max(floor, lo + 1) &&
+                          (rec[i - 1 - lane] & kRecArrival) == uint32_t(j - 1 - lane);
+        const uint32_t hit = __ballot_sync(0xffffffffu, same);
+        const int q = hit ? __ffs(hit) : p;
+        if (lane < q) rec[i - lane] = (lane == 0 ? arrival : uint32_t(j - lane)) | kLeaveDiag;
+        if (hit) return {0u, 0, true};
+        i -= p;
+        j -= p;
+        arrival = uint32_t(j);
+        if (i == lo) break;
+        pl.set_row(i);
+      } else if (hd == kDirStop) {
+        if (lane == 0) rec[i] = arrival | kLeaveStop;
+        return {kExitStop | (local ? 0u : kExitBad) | uint32_t(j), i, false};
+      } else {
+        state = hd;
+      }
+    } else {
+      // E and F runs end inside the matrix; if the planes say otherwise, stop.
+      if (j <= 0) return {kExitBad | kExitStop, i, false};
+      const int d = pl.nib(j);
+      if (state == 1) {
+        --j;
+        if (d & 4) state = 0;
+      } else {
+        if (lane == 0) rec[i] = arrival | kLeaveUp;
+        --i;
+        if (d & 8) state = 0;
+        arrival = uint32_t(j) | uint32_t(state) << 20;
+        if (i == lo) break;
+        if (i >= floor && (rec[i] & kRecArrival) == arrival) return {0u, 0, true};
+        pl.up();
+      }
+    }
+  }
+  return {arrival, lo + 1, false};
+}
+
+template <int R>
+__global__ void __launch_bounds__(kMaxSegs * 32) walk_block_kernel(const WalkArgs A) {
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  __shared__ uint32_t s_entry[kMaxSegs], s_exit[kMaxSegs];
+  __shared__ int s_floor[kMaxSegs];
+  __shared__ int s_cols[kMaxSegs], s_ident[kMaxSegs];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int q = blockIdx.x;
+  const int p = A.tasks[q];
+  ResultDev &res = A.res[p];
+  if (res.status != TSQ_OK) return;
+  const PairDev pr = A.pairs[p];
+  const int m = pr.a_len, n = pr.b_len;
+  const bool local = A.local != 0, emit = A.emit != 0;
+  if (local && res.score <= 0) {
+    if (threadIdx.x == 0) {
+      res.a_begin = res.a_end = res.b_begin = res.b_end = 0;
+      res.n_ident = res.n_cols = 0;
+    }
+    return;
+  }
+  const int ie = local ? res.a_end : m, je = local ? res.b_end : n;
+  // Records of rows 0..ie: shared memory where they fit.
+  uint32_t *rec = ie < A.rec_words ? s_dyn + warps * kWinWords
+                                   : reinterpret_cast<uint32_t *>(A.rec_rows + A.rec_off[q]);
+  using Plane = WarpPlane<R, R == 4 ? kWinSteps4 : kWinSteps8, R == 4 ? kWinLanes4 : kWinLanes8>;
+  static_assert(Plane::kWords <= kWinWords, "windows fit");
+  const int G = A.shape_G[p];
+  Plane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_dyn + w * kWinWords,
+           Plane::band_words(n, G), 31 - __clz(G), lane};
+  const int segs = max(1, min(warps, ie / kSegRows));
+  auto row_of = [&](int k) { return int(int64_t(ie) * k / segs); };
+  const int lo = w < segs ? row_of(w) : 0, hi = w < segs ? row_of(w + 1) : 0;
+  const bool works = w < segs && ie > 0;
+
+  // ---- the path ----
+  auto store = [&](uint32_t entry, const SegWalk &r) {
+    if (lane == 0) {
+      s_entry[w] = entry;
+      if (!r.met) {
+        s_exit[w] = r.exit;
+        s_floor[w] = r.floor;
+      }
+    }
+  };
+  if (works) {
+    int j = je;
+    if (w < segs - 1) j = max(local ? je - (ie - hi) : int(int64_t(je) * hi / ie), min(je, 1));
+    store(uint32_t(j), walk_segment(pl, rec, hi, lo, j, 0, local, hi + 1, lane));
+  }
+  __syncthreads();
+  for (int round = 0; round < segs; ++round) {
+    const uint32_t entry = works && w < segs - 1 ? s_exit[w + 1] : kExitStop;
+    const bool again = !(entry & kExitStop) && entry != s_entry[w];
+    if (!__syncthreads_or(again)) break;
+    if (again)
+      store(entry, walk_segment(pl, rec, hi, lo, int(entry & kRecCol), int(entry >> 20) & 3, local, s_floor[w], lane));
+    __syncthreads();
+  }
+  // The path ends at (bi, bj), in segment `last`.
+  int last = segs - 1, bi = 0, bj = 0;
+  if (ie > 0) {
+    while (last > 0 && !(s_exit[last] & kExitStop)) --last;
+    const uint32_t exit = s_exit[last];
+    if (exit & kExitBad) {  // cannot happen with valid planes
+      if (threadIdx.x == 0) res.status = TSQ_E_CUDA;
+      return;
+    }
+    if (exit & kExitStop) {
+      bi = s_floor[last];
+      bj = int(exit & kRecCol);
+    } else {
+      if (local) bj = int(exit & kRecCol);
+      if (threadIdx.x == 0) rec[0] = (exit & kRecCol) | kLeaveStop;
+    }
+  } else if (threadIdx.x == 0) {
+    rec[0] = uint32_t(je) | kLeaveStop;
+  }
+  __syncthreads();
+
+  // ---- the columns: rows ie down to bi, an even share per warp ----
+  const int total = ie - bi + 1;
+  const int t0 = int(int64_t(total) * w / warps), t1 = int(int64_t(total) * (w + 1) / warps);
+  // Columns of b against gaps in row i, the column it leaves by (next), how.
+  struct Row {
+    int run, next;
+    uint32_t leave;
+  };
+  auto row = [&](int i) {
+    const uint32_t v = rec[i];
+    Row r;
+    r.leave = v & (kLeaveUp | kLeaveStop);
+    r.next = r.leave == kLeaveStop ? bj : int(rec[i - 1] & kRecCol);
+    r.run = int(v & kRecCol) - r.next - (r.leave == kLeaveDiag ? 1 : 0);
+    return r;
+  };
+  int cols = 0;
+  for (int t = t0 + lane; t < t1; t += 32) {
+    const Row r = row(ie - t);
+    cols += r.run + (r.leave != kLeaveStop ? 1 : 0);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cols += __shfl_xor_sync(0xffffffffu, cols, o);
+  if (lane == 0) s_cols[w] = cols;
+  __syncthreads();
+  int64_t off = 0;  // columns below this warp's rows
+  int length = 0;
+  for (int k = 0; k < warps; ++k) {
+    if (k < w) off += s_cols[k];
+    length += s_cols[k];
+  }
+  const int64_t cap = (int64_t)m + n;
+  char *end_a = emit ? A.aln + A.aln_off[p] + cap - 1 : nullptr, *end_b = emit ? end_a + cap : nullptr;
+  const uint8_t *sa = A.seqs + pr.a_off, *sb = A.seqs + pr.b_off;
+  int ident = 0;
+  for (int t = t0; t < t1; t += 32) {
+    const int i = ie - t - lane;
+    Row r{0, 0, kLeaveStop};
+    if (t + lane < t1) r = row(i);
+    const int c = r.run + (r.leave != kLeaveStop ? 1 : 0);
+    int sum = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      sum += lane >= o ? v : 0;
+    }
+    const int64_t pos = off + sum - c;
+    off += __shfl_sync(0xffffffffu, sum, 31);
+    if (r.leave != kLeaveStop) {
+      const uint8_t ca = sa[i - 1], cb = r.leave == kLeaveDiag ? sb[r.next] : uint8_t('-');
+      ident += r.leave == kLeaveDiag && ca == cb;
+      if (emit) {
+        end_a[-(pos + r.run)] = char(ca);
+        end_b[-(pos + r.run)] = char(cb);
+      }
+    }
+    if (!emit) continue;
+    // Gaps in a: short ones by their lane, long ones by the warp.
+    const int top = r.next + r.run + (r.leave == kLeaveDiag ? 1 : 0);  // the arrival column
+    if (r.run <= 32)
+      for (int x = 0; x < r.run; ++x) {
+        end_a[-(pos + x)] = '-';
+        end_b[-(pos + x)] = char(sb[top - 1 - x]);
+      }
+    for (uint32_t far = __ballot_sync(0xffffffffu, r.run > 32); far; far &= far - 1) {
+      const int k = __ffs(far) - 1;
+      const int run = __shfl_sync(0xffffffffu, r.run, k), from = __shfl_sync(0xffffffffu, top, k);
+      const int64_t at = __shfl_sync(0xffffffffu, pos, k);
+      for (int x = lane; x < run; x += 32) {
+        end_a[-(at + x)] = '-';
+        end_b[-(at + x)] = char(sb[from - 1 - x]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ident += __shfl_xor_sync(0xffffffffu, ident, o);
+  if (lane == 0) s_ident[w] = ident;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  ident = 0;
+  for (int k = 0; k < warps; ++k) ident += s_ident[k];
+  if (emit || !local) {
+    res.a_begin = bi;
+    res.b_begin = bj;
+  }
+  if (!local) {
+    res.a_end = m;
+    res.b_end = n;
+  }
+  res.n_cols = length;
+  res.n_ident = ident;
 }
 
 // ASCII -> letter codes, and (when clut is set) -> score classes for the
@@ -371,6 +647,26 @@ cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st) {
     walk_warp_kernel<true><<<blocks, kWarpWalkWarps * 32, 0, st>>>(a);
   else
     walk_warp_kernel<false><<<blocks, kWarpWalkWarps * 32, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+// Warps of the many-warps walk: a segment each of at least kSegRows rows, and
+// over all pairs about two warps for every place on the GPU.
+cudaError_t launch_walk_block(const WalkArgs &args, int R, int32_t max_rows, cudaStream_t st) {
+  if (args.n_tasks <= 0) return cudaSuccess;
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int share = std::max(4, sms * kMaxSegs * 2 / args.n_tasks);
+  const int warps = std::max(1, std::min({kMaxSegs, share, max_rows / kSegRows}));
+  const size_t windows = size_t(warps) * kWinWords * 4;
+  WalkArgs a = args;
+  a.rec_words = int32_t(std::min<size_t>((kWalkSmem - windows) / 4, size_t(max_rows) + 1));
+  const size_t smem = windows + size_t(a.rec_words) * 4;
+  auto kernel = R == 4 ? walk_block_kernel<4> : walk_block_kernel<8>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kWalkSmem));
+  if (e != cudaSuccess) return e;
+  kernel<<<a.n_tasks, warps * 32, smem, st>>>(a);
   return cudaGetLastError();
 }
 
