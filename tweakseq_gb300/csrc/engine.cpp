@@ -722,6 +722,11 @@ int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts
   return TSQ_OK;
 }
 
+// Pairs of a strip launch up to which each is walked by a block's warps: 20 pairs
+// x 3,000 0.17 -> 0.05 ms, 300 x 3,000 0.20 -> 0.09, 300 x 1,200 0.10 -> 0.07; with
+// more, a warp for each pair fills the GPU and walks no cell twice.
+constexpr int32_t kManyWalks = 1024;
+
 // A pair is long when its sweep on one 32-lane group takes more steps than
 // kLongSteps and kLongShare of the batch's balanced per-lane work.  Device
 // time of protein batches (log-normal lengths, median as named), shares of
@@ -732,10 +737,6 @@ int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts
 // warp is as fast as strips up to about 600 steps (20 pairs x 150: 0.067 ms
 // either way).  Identity output's long form is a CTA of 8 warps, worth its
 // int32 cells from 20,000 steps.
-// Pairs of a strip launch up to which each is walked by a block's warps: 20 pairs
-// x 3,000 0.17 -> 0.05 ms, 300 x 3,000 0.20 -> 0.09, 300 x 1,200 0.10 -> 0.07; with
-// more, a warp for each pair fills the GPU and walks no cell twice.
-constexpr int32_t kManyWalks = 1024;
 constexpr double kLongSteps = 600.0, kLongShare = 1.5, kLongStepsCta = 20000.0;
 
 // The strip launch of the pairs at [s, e) of the sorted order: its units,
@@ -779,7 +780,8 @@ void plan_strips(tsq_batch *b, PlanScratch &ps, int64_t s, int64_t e, StripKind 
   for (const SortRec &r : key) units->push_back(list[size_t(r.idx)]);
   L.n_wtasks = int32_t(list.size());
   const int max_blocks = strip_blocks(kind, b->fill_mode, b->local, b->scheme.nclasses);
-  L.blocks = int32_t(std::min<int64_t>(max_blocks, L.n_wtasks));
+  const bool beside = e - s < b->n;  // other fills run at the same time
+  L.blocks = int32_t(std::min<int64_t>(beside ? std::max(1, max_blocks / 2) : max_blocks, L.n_wtasks));
   b->strip_clear = size_t(L.n_pairs) * sizeof(StripCtl) + size_t(entries) * 8;
   b->launches.push_back(L);
 }

@@ -86,6 +86,13 @@ StripKind StripLoad::pick(int out_mode, int sms, bool allow16) const {
   return best;
 }
 
+// Blocks (warps) of a strip launch: two on each scheduler, one beside other fills.
+// Device time of the fills, ms, with as many as fit (2.5 a scheduler and more,
+// unevenly spread) / two / one: 23 DNA pairs of 10 to 50 kb with traceback 25.0 /
+// 22.8 / 24.2, score 11.3 / 10.8 / 12.3, 200 of 3 to 9 kb 5.6 / 5.1 / 5.8; strips
+// beside short pairs, 1,000 proteins of median 800 1.48 / 1.48 / 1.05, 60 of median
+// 4,000 5.1 / 3.7 / 3.4.  Two warps fill a scheduler; a third only lengthens the
+// steps of the longest pair's chain, and an uneven spread lengthens some.
 int strip_blocks(StripKind kind, int out_mode, bool local, int nclasses) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -100,8 +107,10 @@ int strip_blocks(StripKind kind, int out_mode, bool local, int nclasses) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const fill::Kernel k = fill::strip_kernel(kind, out_mode, local);
   int nb = 0;
+  constexpr int kSchedulers = 4;
   if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32, fill::strip_smem(kind, nclasses)) != cudaSuccess)
     return 0;
+  nb = std::min(nb, 2 * kSchedulers);
   if (nb * sms > 0) {
     std::lock_guard<std::mutex> g(mu);
     known[key] = nb * sms;
