@@ -21,7 +21,9 @@
 // row's F.  F can take X instead of H from the row above because open >= 0
 // makes the F - open - ext candidate redundant, so rows depend on each other
 // through one add-max only.  (Local score launches have a shorter form: TD
-// below.)
+// below.  The traceback fill takes F from H, which saves the second subtraction
+// and, in global mode, X: H = max(D + s, E, F).  20,000 pairs of 350 x 350 1.385
+// -> 1.328 ms, 10,000 of 500 x 500 1.348 -> 1.289.)
 //
 // Biased halves.  Every value v is held as v + 32768 in an unsigned 16-bit
 // half, compared with the unsigned DPX forms; the proven range keeps every
@@ -48,12 +50,12 @@
 // the values (even in halves outside their column range), and one 32-bit
 // subtraction computes both without a borrow crossing the halves;
 // min(difference, 1) per half is then the decision bit of each cell.  With
-// open >= 0 the F decision taken from X instead of H differs from the
+// open >= 0 an F decision taken from X instead of H (identity) differs from the
 // int32 fill's only when open = 0 and F beats X strictly; both then walk
 // through the same cells and count the same columns.
 //
-// Traceback: per row, the nibble dir | E-open << 2 | F-open << 3 (dir =
-// [h > dd] + [h > x], or 3 for a local stop) is summed into two words by
+// Traceback: per row, the nibble dir | E-open << 2 | F-open << 3 (dir:
+// local [h > dd] + [h > x], or 3 for a stop; global [h > dd] + 2 [h > e]) is summed into two words by
 // integer multiply-adds (rows 0-3 and 4-7, band A in the low halves, band
 // B in the high halves), and two PRMTs give each band's 32-bit plane word.
 // The planes have the int32 fill's layout -- band A of pass p is band 2p,
@@ -601,14 +603,18 @@ __device__ __forceinline__ void fill16_warp_task(const FillArgs &A, const int8_t
             }
             const uint32_t fo = r == 0 ? xo0 : xo;  // F's open candidate
             const uint32_t f = r == 0 ? fv : __viaddmax_u16x2(fv, nge2, xo);
-            uint32_t h = LOCAL ? __vimax3_u16x2(x, f, kBias2) : __vimax3_u16x2(x, f, f);
+            uint32_t h = LOCAL                ? __vimax3_u16x2(x, f, kBias2)
+                         : OUT == kOutTrace ? __vimax3_u16x2(dd, e, f)
+                                            : __vimax3_u16x2(x, f, f);
             uint32_t tn = sub2_imad(h, one, neg_oe2);
-            xo = LOCAL ? __viaddmax_u16x2(x, noe2, zero_oe2) : sub2_imad(x, one, neg_oe2);
+            // (Traceback: from H; its many decisions hide the longer chain.)
+            xo = OUT == kOutTrace ? tn : LOCAL ? __viaddmax_u16x2(x, noe2, zero_oe2) : sub2_imad(x, one, neg_oe2);
             (void)fo;
             if constexpr (OUT == kOutTrace) {
-              // dir = [h > dd] + [h > x]; bits 2 and 3 clear when E / F
-              // extended.
-              uint32_t c = imad(nz2(h, x, minus_one, k1), one, nz2(h, dd, minus_one, k1));
+              // Local: dir = [h > dd] + [h > x].  Global: [h > dd], [h > e].
+              // Bits 2 and 3 clear when E / F extended.
+              uint32_t c = LOCAL ? imad(nz2(h, x, minus_one, k1), one, nz2(h, dd, minus_one, k1))
+                                 : imad(nz2(h, e, minus_one, k1), one + one, nz2(h, dd, minus_one, k1));
               c = imad(nz2(e, T[r], minus_one, k1), m4, c);
               c = imad(nz2(f, fo, minus_one, k1), m8, c);
               const uint32_t w = (r & 3) == 0 ? one : (r & 3) == 1 ? k16 : (r & 3) == 2 ? k256 : k4096;

@@ -268,7 +268,7 @@ __device__ __forceinline__ void fill_warp_task(const FillArgs &A, const int8_t *
               bool pde, pxf;
               const int32_t x = max_pred(dd, e, &pde);
               h = max_pred(x, f, &pxf);
-              int dir = pxf ? (pde ? int(kDirDiag) : int(kDirE)) : int(kDirF);
+              int dir = pxf ? (pde ? int(kDirDiag) : int(kDirE)) : LOCAL ? int(kDirF) : int(kDirFGlobal);
               if (LOCAL && h <= 0) {
                 h = 0;
                 dir = kDirStop;

@@ -158,12 +158,11 @@ __global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
       // The warp's values are relative to bw (absolute); it starts at the
       // strip's top-left cell H(512p, 0).
       int32_t bw = edge_h(strip * P2, go, ge, LOCAL);
-      // Local: H's floor 0, and 0 - open - ext, on the warp's scale.
-      uint32_t zero2 = 0u, zero_oe2 = 0u;
+      // Local: H's floor 0 on the warp's scale.
+      uint32_t zero2 = 0u;
       auto set_zero = [&]() {
-        const uint32_t z = uint32_t(max(-bw, kNeg16) + kBias16), zo = uint32_t(max(-bw - oe, kNeg16) + kBias16);
+        const uint32_t z = uint32_t(max(-bw, kNeg16) + kBias16);
         zero2 = (z << 16) | z;
-        zero_oe2 = (zo << 16) | zo;
       };
       if constexpr (LOCAL) set_zero();
       uint32_t H[R], E[R], T[R];
@@ -350,18 +349,24 @@ __global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
                 x = __viaddmax_u16x2(d, sc, e);
               } else {
                 dd = __viaddmax_u16x2(d, sc, 0u);  // D + s per half
-                x = __vimax3_u16x2(dd, e, e);
+                x = LOCAL ? __vimax3_u16x2(dd, e, e) : 0u;
               }
               const uint32_t fo = r == 0 ? xo0 : xo;  // F's open candidate
               const uint32_t f = r == 0 ? fv : __viaddmax_u16x2(fv, nge2, xo);
-              uint32_t h = LOCAL ? __vimax3_u16x2(x, f, zero2) : __vimax3_u16x2(x, f, f);
+              uint32_t h = LOCAL                ? __vimax3_u16x2(x, f, zero2)
+                           : OUT == kOutTrace ? __vimax3_u16x2(dd, e, f)
+                                              : __vimax3_u16x2(x, f, f);
               uint32_t tn = sub2_imad(h, one, neg_oe2);
-              xo = LOCAL ? __viaddmax_u16x2(x, noe2, zero_oe2) : sub2_imad(x, one, neg_oe2);
+              // (From H where a step has decisions or maxima enough to hide the
+              // longer chain: 23 pairs of 10 to 50 kb with traceback 23.2 -> 20.7 ms,
+              // local scores 19.4 -> 17.5; global scores 10.4 -> 11.6, not taken.)
+              xo = OUT == kOutTrace || LOCAL ? tn : sub2_imad(x, one, neg_oe2);
               (void)fo;
               if constexpr (OUT == kOutTrace) {
-                // dir = [h > dd] + [h > x]; bits 2 and 3 clear when E / F
-                // extended.
-                uint32_t c = imad(nz2(h, x, minus_one, k1), one, nz2(h, dd, minus_one, k1));
+                // Local: dir = [h > dd] + [h > x].  Global: [h > dd], [h > e].
+                // Bits 2 and 3 clear when E / F extended.
+                uint32_t c = LOCAL ? imad(nz2(h, x, minus_one, k1), one, nz2(h, dd, minus_one, k1))
+                                   : imad(nz2(h, e, minus_one, k1), one + one, nz2(h, dd, minus_one, k1));
                 c = imad(nz2(e, T[r], minus_one, k1), m4, c);
                 c = imad(nz2(f, fo, minus_one, k1), m8, c);
                 const uint32_t wgt = (r & 3) == 0 ? one : (r & 3) == 1 ? k16 : (r & 3) == 2 ? k256 : k4096;

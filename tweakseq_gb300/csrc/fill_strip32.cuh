@@ -8,7 +8,7 @@
 // in about 2.3 cycles whatever is independent (two columns a step, to fill
 // waits, only made the strips start further apart: 2.33 against 1.94 ms on
 // 20,000 x 20,000, score), so what counts is the instructions of a step.  Per
-// cell the score fill issues 7, the traceback fill 16: each of the four
+// cell the score fill issues 7, the traceback fill 14: each of the four
 // decisions is the sign of one difference (an IMAD by an opaque -1, FMA
 // pipe), shifted into a word by one funnel shift.  Beside its cells a step
 // issues about 17: the shuffles that join the lanes, the code, profile and
@@ -19,7 +19,7 @@
 // rows, step s = column + lane: lane t at word
 // (b * ceil((n + 31) / 2) + s / 2) * 32 + t, row r of step s in nibble
 // 7 - (s % 2 * 4 + r), the nibble as in the other fills (bits 0-1 direction,
-// 3 a local stop; bit 2 E opened, bit 3 F opened).
+// bit 2 E opened, bit 3 F opened).
 #pragma once
 
 #include <algorithm>
@@ -199,22 +199,29 @@ __global__ void __launch_bounds__(32) fill_strip32_kernel(const FillArgs A) {
             const int32_t sc = sbyte_dyn(w, r);
             const int32_t e = __viaddmax_s32(E[r], -ge, T[r]);
             const int32_t f = __viaddmax_s32(fv, -ge, xo);
-            int32_t x, h;
+            int32_t x = 0, h;
             if constexpr (OUT == kOutScore) {
               x = __viaddmax_s32(d, sc, e);
               h = LOCAL ? __vimax3_s32(x, f, 0) : max(x, f);
             } else {
               const int32_t dd = mad(sc, one, d);
-              x = max(dd, e);
-              h = LOCAL ? __vimax3_s32(x, f, 0) : max(x, f);
+              x = LOCAL ? max(dd, e) : 0;
+              h = LOCAL ? __vimax3_s32(x, f, 0) : __vimax3_s32(dd, e, f);
               acc = push_sign(acc, mad(f, minus_one, xo));    // F extended
               acc = push_sign(acc, mad(e, minus_one, T[r]));  // E extended
-              acc = push_sign(acc, mad(h, minus_one, x));     // H not from X
-              acc = push_sign(acc, mad(x, minus_one, dd));    // X from E
+              if constexpr (LOCAL) {
+                acc = push_sign(acc, mad(h, minus_one, x));   // H not from X
+                acc = push_sign(acc, mad(x, minus_one, dd));  // X from E
+              } else {
+                acc = push_sign(acc, mad(h, minus_one, e));   // H above E
+                acc = push_sign(acc, mad(h, minus_one, dd));  // H not the diagonal's
+              }
               if constexpr (LOCAL) stop |= uint32_t((h - 1) >> 31) & (3u << (4 * (7 - ((k % U) * R + r))));
             }
-            xo = LOCAL ? __viaddmax_s32(x, -oe, -oe) : mad(x, one, -oe);
             T[r] = mad(h, one, -oe);
+            // (Score: from X, a shorter chain through the rows: one pair of 20 kb
+            // 1.86 ms, from H 2.05.)
+            xo = OUT == kOutTrace ? T[r] : LOCAL ? __viaddmax_s32(x, -oe, -oe) : mad(x, one, -oe);
             E[r] = e;
             d = H[r];
             H[r] = h;
@@ -232,9 +239,9 @@ __global__ void __launch_bounds__(32) fill_strip32_kernel(const FillArgs A) {
         }
         if (t == 31) outp[k] = make_int2(outH, outF);
         if constexpr (OUT == kOutTrace && k % U == U - 1) {
-          // dir: E only where F does not win; the opened bits are the
+          // Local: E only where F does not win.  The opened bits are the
           // complements of the extended ones.
-          uint32_t word = (acc & ~((acc >> 1) & 0x11111111u)) ^ 0xCCCCCCCCu;
+          uint32_t word = (LOCAL ? acc & ~((acc >> 1) & 0x11111111u) : acc) ^ 0xCCCCCCCCu;
           if constexpr (LOCAL) {
             word |= stop;
             stop = 0u;

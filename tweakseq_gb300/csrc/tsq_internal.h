@@ -37,6 +37,10 @@ constexpr int64_t kMaxPairLen = (1 << 20) - 1;
 enum : int { kOutScore = 0, kOutIdent = 1, kOutTrace = 2 };
 // Traceback nibble: bits 0-1 H source, bit 2 E opened, bit 3 F opened.
 enum : int { kDirDiag = 0, kDirE = 1, kDirF = 2, kDirStop = 3 };
+// The two low bits of a cell in the traceback planes.  Local: one of the above.
+// Global: bit 0 H is not the diagonal's, bit 1 H is above E, so 0 and 2 stand for
+// the diagonal, 1 for E and 3 for F (a bit less to work out per cell).
+constexpr int kDirFGlobal = 3;
 
 struct Scheme {
   int8_t score[kLetters][kLetters];

@@ -51,7 +51,7 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
     }
     if (state == 0) {
       if (A.local) {
-        if (i == 0 || j == 0 || (pl.nib(j) & 3) == kDirStop) break;
+        if (i == 0 || j == 0 || pl.dir(j) == kDirStop) break;
       } else if (i == 0 && j == 0) {
         break;
       }
@@ -104,7 +104,7 @@ __device__ __forceinline__ void walk_pair(const WalkArgs &A, const PairDev &pr, 
         if (i > 0) pl.up();
         continue;
       }
-      const int hd = pl.nib(j) & 3;
+      const int hd = pl.dir(j);
       if (hd == kDirDiag) {
         ++L;
         const uint8_t ca = a.at(i - 1), cb = b.at(j - 1);
@@ -189,6 +189,7 @@ struct WarpPlane {
   uint32_t *win;  // kWords words of this warp
   int row_words;  // words of a band per lane
   int gshift, lane;
+  uint32_t diag_bits;  // bits that are 0 where H is the diagonal's: 3 local, 1 global
   int g = 0, r = 0;
   int wg = -1, ws = -1;
   static __device__ int band_words(int n, int G) { return (n + G - 1 + (1 << kUShift) - 1) >> kUShift; }
@@ -231,6 +232,12 @@ struct WarpPlane {
     if (g > wg || g <= wg - WL || s > ws || s <= ws - WS) refill(s);
     return int(win[(ws - s) * WL + (wg - g)] >> shift_of(q, r)) & 15;
   }
+  // Where H of the cell comes from.
+  __device__ int dir(int j) {
+    const int v = nib(j);
+    if ((uint32_t(v) & diag_bits) == 0u) return kDirDiag;
+    return diag_bits == 3u ? v & 3 : (v & 2 ? kDirF : kDirE);
+  }
   // Lanes whose cell (i - lane, j - lane) lies inside the matrix and the
   // current window and takes H from the diagonal.
   __device__ uint32_t diag_mask(int i, int j) const {
@@ -240,7 +247,7 @@ struct WarpPlane {
       const int gk = (ik - 1) >> kRShift, rk = (ik - 1) & (R - 1);
       const int q = jk - 1 + gk, sk = q >> kUShift;
       if (gk > wg - WL && sk > ws - WS)
-        d = ((win[(ws - sk) * WL + (wg - gk)] >> shift_of(q, rk)) & 3) == uint32_t(kDirDiag);
+        d = ((win[(ws - sk) * WL + (wg - gk)] >> shift_of(q, rk)) & diag_bits) == 0u;
     }
     return __ballot_sync(0xffffffffu, d);
   }
@@ -289,7 +296,7 @@ __device__ __forceinline__ void walk_one(const WalkArgs &A, int p, uint32_t *s_p
   char *out_a = A.emit ? A.aln + A.aln_off[p] : nullptr;
   const int G = A.shape_G[p];
   Plane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_plane,
-           Plane::band_words(pr.b_len, G), 31 - __clz(G), lane};
+           Plane::band_words(pr.b_len, G), 31 - __clz(G), lane, A.local ? 3u : 1u};
   walk_pair(A, pr, res, pl, a, b, out_a, out_a + cap, cap, lane);
 }
 
@@ -383,7 +390,7 @@ __device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi
         for (int k = i - lane; k > lo; k -= 32) rec[k] = (k == i ? arrival : 0u) | kLeaveUp;
         return {0u, lo + 1, false};
       }
-      const int hd = pl.nib(j) & 3;
+      const int hd = pl.dir(j);
       if (hd == kDirDiag) {
         // A run of diagonal moves at once: lane k leaves row i - k.
         const uint32_t dm = pl.diag_mask(i, j);
@@ -456,7 +463,7 @@ __global__ void __launch_bounds__(kMaxSegs * 32) walk_block_kernel(const WalkArg
   static_assert(Plane::kWords <= kWinWords, "windows fit");
   const int G = A.shape_G[p];
   Plane pl{reinterpret_cast<const uint32_t *>(A.planes + A.plane_off[p]), s_dyn + w * kWinWords,
-           Plane::band_words(n, G), 31 - __clz(G), lane};
+           Plane::band_words(n, G), 31 - __clz(G), lane, local ? 3u : 1u};
   const int segs = max(1, min(warps, ie / kSegRows));
   auto row_of = [&](int k) { return int(int64_t(ie) * k / segs); };
   const int lo = w < segs ? row_of(w) : 0, hi = w < segs ? row_of(w + 1) : 0;
