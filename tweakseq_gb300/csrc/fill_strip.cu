@@ -118,13 +118,13 @@ int strip_blocks(StripKind kind, int out_mode, bool local, int nclasses) {
   return nb * sms;
 }
 
-cudaError_t launch_strip(StripKind kind, int out_mode, bool local, const FillArgs &args, int blocks, cudaStream_t st) {
+cudaError_t launch_strip(StripKind kind, int out_mode, bool local, const FillArgs &args, int blocks, cudaStream_t st,
+                         bool early) {
   const fill::Kernel k = fill::strip_kernel(kind, out_mode, local);
   if (!k) return cudaErrorInvalidValue;
   FillArgs a = args;
   a.one = 1u;
-  k<<<blocks, 32, fill::strip_smem(kind, a.nclasses), st>>>(a);
-  return cudaGetLastError();
+  return launch_maybe_early(k, dim3(blocks), 32, fill::strip_smem(kind, a.nclasses), st, early, a);
 }
 
 }  // namespace tsq

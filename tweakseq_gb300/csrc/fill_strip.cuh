@@ -46,6 +46,13 @@ namespace fill {
 constexpr uint32_t kTagMask = 0x3FFFu;  // tags 1..16383
 static_assert((kMaxPairLen + 127) / 128 - 1 <= int64_t(kTagMask), "a tag for every strip that hands down");
 
+// Lets the next launch start (it waits for this one), and waits for the one ahead,
+// where the launches allow it (launch_maybe_early).
+__device__ __forceinline__ void strip_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t strip_tag(int strip) { return uint32_t(strip) + 1u; }
 
 // (H, F) of a bottom-row cell as a tagged entry; dmax = open + 1.

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
   constexpr int G = 32, R = 8, P = G * R, P2 = 2 * P, C = kStripCols16;
   constexpr int kThr = 32;
   extern __shared__ __align__(16) uint8_t smem[];
+  strip_begin();
   int8_t *s_mat = reinterpret_cast<int8_t *>(smem);
   uint2 *s_prof = reinterpret_cast<uint2 *>(smem + kMatBytes16);
   const int ncls = A.nclasses;

@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(32) fill_strip32_kernel(const FillArgs A) {
   static_assert(OUT == kOutScore || OUT == kOutTrace, "score and traceback output");
   constexpr int R = 4, S = kStripRows32, C = kStripCols32, U = 8 / R;  // U: steps per plane word
   extern __shared__ __align__(16) uint8_t smem[];
+  strip_begin();
   int8_t *s_mat = reinterpret_cast<int8_t *>(smem);
   uint32_t *s_prof = reinterpret_cast<uint32_t *>(smem + kMatBytes16);
   const int ncls = A.nclasses;

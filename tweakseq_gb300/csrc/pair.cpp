@@ -128,7 +128,7 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   const int64_t off_bnd = off_res + align256(down_bytes);
   // The strips' hand-over row, later the walk's records where those need it.
   int64_t bnd_bytes = n_units > 1 ? (int64_t(lb) + 15) / 16 * 16 * 8 : 0;
-  if (out_mode != kOutScore && la >= kWalkRecRows) bnd_bytes = std::max(bnd_bytes, (int64_t(la) + 2) / 2 * 8);
+  if (out_mode != kOutScore && la >= kWalkRecRows) bnd_bytes = std::max(bnd_bytes, (int64_t(la) + 3) / 4 * 16);
   const int64_t off_planes = off_bnd + align256(bnd_bytes);
   const int64_t plane_total = walk ? plane_bytes(la, lb, shp) : 0;
   const int64_t dev_bytes = off_planes + std::max<int64_t>(plane_total, 16);
@@ -165,7 +165,9 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   uint8_t *ccodes = d + off_ccodes;
   ResultDev *res = reinterpret_cast<ResultDev *>(d + off_res);
   PAIR_TRY(cudaMemcpyAsync(d, h, size_t(up_bytes), cudaMemcpyHostToDevice, st));
-  PAIR_TRY(launch_encode(seqs, len + kPad, d + kOffLut, codes, d + kOffClut, ccodes, st));
+  // (It also clears the hand-over row, and the launches after it start early: the
+  // gaps between a short pair's launches are a tenth of its call.)
+  PAIR_TRY(launch_encode(seqs, len + kPad, d + kOffLut, codes, d + kOffClut, ccodes, st, d + off_bnd, bnd_bytes));
 
   // ---- fill ----------------------------------------------------------------
   FillArgs fa{};
@@ -188,8 +190,7 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   fa.strip_ctl = reinterpret_cast<StripCtl *>(d + kOffCtl);
   fa.strip_rows = reinterpret_cast<uint64_t *>(d + off_bnd);
   fa.strip_row_off = reinterpret_cast<const int64_t *>(d + kOffRowOff);
-  if (bnd_bytes > 0) PAIR_TRY(cudaMemsetAsync(d + off_bnd, 0, size_t(bnd_bytes), st));
-  PAIR_TRY(launch_strip(kind, fill_mode, local, fa, std::min(blocks_avail, n_units), st));
+  PAIR_TRY(launch_strip(kind, fill_mode, local, fa, std::min(blocks_avail, n_units), st, true));
 
   // ---- traceback ---------------------------------------------------------
   char *rows = reinterpret_cast<char *>(d + off_res + sizeof(ResultDev));
@@ -211,7 +212,7 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
     w.aln_off = reinterpret_cast<const int64_t *>(d + kOffAlnOff);
     w.rec_rows = fa.strip_rows;
     w.rec_off = fa.strip_row_off;
-    PAIR_TRY(launch_walk_block(w, shp.R, la, st));
+    PAIR_TRY(launch_walk_block(w, shp.R, la, st, true));
   }
   PAIR_TRY(cudaMemcpyAsync(pp->down.p, res, size_t(down_bytes), cudaMemcpyDeviceToHost, st));
   PAIR_TRY(cudaStreamSynchronize(st));

@@ -157,6 +157,23 @@ void build_lut(const Scheme &s, uint8_t lut[256]);
 // code marks invalid).
 void build_class_lut(const Scheme &s, uint8_t lut[256]);
 
+// A launch that may (early) start before the one ahead of it in the stream ends.
+template <class Args>
+cudaError_t launch_maybe_early(void (*kernel)(const Args), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                               bool early, const Args &args) {
+  cudaLaunchAttribute attr[1] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 // Kernel launchers (fill_dispatch.cu, fill_i16.cu, fill_cta.cu, walk_kernel.cu).
 // Returns the number of thread blocks a persistent launch of this shape uses.
 // A launch covers every lane width G of one row height R and lane type
@@ -187,7 +204,10 @@ bool strip16_supported(const Scheme &sc, int32_t gap_open, int32_t gap_extend);
 int strip_rows(StripKind kind);
 Shape strip_shape(StripKind kind);  // of the traceback planes
 int strip_blocks(StripKind kind, int out_mode, bool local, int nclasses);
-cudaError_t launch_strip(StripKind kind, int out_mode, bool local, const FillArgs &a, int blocks, cudaStream_t st);
+// early: may start before the launch ahead of it in the stream ends (which must
+// be one that lets it: launch_encode, launch_strip); the kernel waits for it.
+cudaError_t launch_strip(StripKind kind, int out_mode, bool local, const FillArgs &a, int blocks, cudaStream_t st,
+                         bool early = false);
 // The work of a set of pairs in each kind of strips, and the kind that is
 // estimated to finish first: the longer of its longest pair's chain of steps
 // and its total steps over all schedulers.
@@ -201,13 +221,13 @@ cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st);
 // The pairs of a strip launch, one block each; max_rows: their longest a.
 // Pairs of at least kWalkRecRows rows need room for their records.
 constexpr int32_t kWalkRecRows = 32768;
-cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st);
-// The pairs of a strip launch, one block each; max_rows: their longest a.
-cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st);
+cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st, bool early = false);
 // Residues -> letter codes and, when clut_dev / ccodes are set, score
 // classes.
+// zero: zero_bytes (a multiple of 16, 16-byte aligned) that the launch also clears.
 cudaError_t launch_encode(const uint8_t *seqs, int64_t len, const uint8_t *lut_dev, uint8_t *codes,
-                          const uint8_t *clut_dev, uint8_t *ccodes, cudaStream_t st);
+                          const uint8_t *clut_dev, uint8_t *ccodes, cudaStream_t st,
+                          void *zero = nullptr, int64_t zero_bytes = 0);
 
 // Bytes of traceback planes a pair needs under a shape: words of eight cells
 // per lane, R rows (8, or 4 in int32 strips) of 8 / R steps (step = column +

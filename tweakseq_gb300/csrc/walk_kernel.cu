@@ -437,6 +437,7 @@ __device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi
 template <int R>
 __global__ void __launch_bounds__(kMaxSegs * 32) walk_block_kernel(const WalkArgs A) {
   extern __shared__ __align__(16) uint32_t s_dyn[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ uint32_t s_entry[kMaxSegs], s_exit[kMaxSegs];
   __shared__ int s_floor[kMaxSegs];
   __shared__ int s_cols[kMaxSegs], s_ident[kMaxSegs];
@@ -611,7 +612,8 @@ __global__ void __launch_bounds__(kMaxSegs * 32) walk_block_kernel(const WalkArg
 // int16x2 fill, through shared-memory tables.
 __global__ void encode_kernel(const uint8_t *__restrict__ seqs, int64_t len, const uint8_t *__restrict__ lut,
                               uint8_t *__restrict__ codes, const uint8_t *__restrict__ clut,
-                              uint8_t *__restrict__ ccodes) {
+                              uint8_t *__restrict__ ccodes, uint4 *__restrict__ zero, int64_t nzero) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ uint8_t s_lut[256], s_clut[256];
   s_lut[threadIdx.x] = lut[threadIdx.x];
   s_clut[threadIdx.x] = clut ? clut[threadIdx.x] : uint8_t(0);
@@ -623,6 +625,8 @@ __global__ void encode_kernel(const uint8_t *__restrict__ seqs, int64_t len, con
   uint4 *dst = reinterpret_cast<uint4 *>(codes);
   uint4 *cdst = reinterpret_cast<uint4 *>(ccodes);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nzero; v += stride)
+    zero[v] = make_uint4(0u, 0u, 0u, 0u);
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += stride) {
     const uint4 w0 = src[v];
     uint4 w = w0, c = w0;
@@ -659,7 +663,7 @@ cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st) {
 
 // Warps of the many-warps walk: a segment each of at least kSegRows rows, and
 // over all pairs about two warps for every place on the GPU.
-cudaError_t launch_walk_block(const WalkArgs &args, int R, int32_t max_rows, cudaStream_t st) {
+cudaError_t launch_walk_block(const WalkArgs &args, int R, int32_t max_rows, cudaStream_t st, bool early) {
   if (args.n_tasks <= 0) return cudaSuccess;
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
@@ -673,20 +677,20 @@ cudaError_t launch_walk_block(const WalkArgs &args, int R, int32_t max_rows, cud
   auto kernel = R == 4 ? walk_block_kernel<4> : walk_block_kernel<8>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kWalkSmem));
   if (e != cudaSuccess) return e;
-  kernel<<<a.n_tasks, warps * 32, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_maybe_early(kernel, dim3(a.n_tasks), warps * 32, smem, st, early, a);
 }
 
 cudaError_t launch_encode(const uint8_t *seqs, int64_t len, const uint8_t *lut_dev, uint8_t *codes,
-                          const uint8_t *clut_dev, uint8_t *ccodes, cudaStream_t st) {
-  if (len <= 0) return cudaSuccess;
+                          const uint8_t *clut_dev, uint8_t *ccodes, cudaStream_t st, void *zero, int64_t zero_bytes) {
+  if (len <= 0 && zero_bytes <= 0) return cudaSuccess;
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t work = (len + 15) / 16;
+  const int64_t work = std::max(len + 15, zero_bytes) / 16;
   int blocks = int(std::min<int64_t>((work + 255) / 256, (int64_t)sms * 8));
   if (blocks < 1) blocks = 1;
-  encode_kernel<<<blocks, 256, 0, st>>>(seqs, len, lut_dev, codes, clut_dev, ccodes);
+  encode_kernel<<<blocks, 256, 0, st>>>(seqs, len, lut_dev, codes, clut_dev, ccodes, static_cast<uint4 *>(zero),
+                                      zero_bytes / 16);
   return cudaGetLastError();
 }
 
