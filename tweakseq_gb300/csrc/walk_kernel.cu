@@ -251,6 +251,20 @@ struct WarpPlane {
     }
     return __ballot_sync(0xffffffffu, d);
   }
+  // Lanes whose cell (i, j - lane) (E) or (i - lane, j) (F) lies inside the
+  // matrix and the current window and extends its gap.
+  template <bool IN_ROW>
+  __device__ uint32_t gap_mask(int i, int j) const {
+    const int ik = IN_ROW ? i : i - lane, jk = IN_ROW ? j - lane : j;
+    bool d = false;
+    if (ik >= 1 && jk >= 1) {
+      const int gk = (ik - 1) >> kRShift, rk = (ik - 1) & (R - 1);
+      const int q = jk - 1 + gk, sk = q >> kUShift;
+      if (gk > wg - WL && sk > ws - WS)
+        d = ((win[(ws - sk) * WL + (wg - gk)] >> shift_of(q, rk)) & (IN_ROW ? 4u : 8u)) == 0u;
+    }
+    return __ballot_sync(0xffffffffu, d);
+  }
 };
 
 // One sequence read backwards through a shared window of WIN residues.
@@ -379,6 +393,22 @@ __device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi
   int i = hi;
   uint32_t arrival = uint32_t(j) | uint32_t(state) << 20;
   pl.set_row(i);
+  // Leaves p rows, each `left` columns further left, arriving in the next with
+  // `st` (the state's bits).  True when one of the rows it arrives in was arrived
+  // in like that before.
+  auto advance = [&](int p, int left, uint32_t st, uint32_t leave) {
+    const int rk = i - 1 - lane;  // arrived in from row i - lane
+    const bool same = lane < p && rk >= max(floor, lo + 1) &&
+                      (rec[rk] & kRecArrival) == (uint32_t(j - left * (lane + 1)) | st);
+    const uint32_t hit = __ballot_sync(0xffffffffu, same);
+    const int q = hit ? __ffs(hit) : p;
+    if (lane < q) rec[i - lane] = (lane == 0 ? arrival : uint32_t(j - left * lane) | st) | leave;
+    i -= p;
+    j -= left * p;
+    arrival = uint32_t(j) | st;
+    if (i > lo) pl.set_row(i);
+    return hit != 0u;
+  };
   for (;;) {
     if (state == 0) {
       if (j == 0) {
@@ -395,18 +425,8 @@ __device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi
         // A run of diagonal moves at once: lane k leaves row i - k.
         const uint32_t dm = pl.diag_mask(i, j);
         const int p = min(dm == 0xffffffffu ? 32 : __ffs(~dm) - 1, i - lo);
-        // Arrivals of rows i - 1 - lane, the run's and the one it leads to.
-        const bool same = lane < p && i - 1 - lane >= max(floor, lo + 1) &&
-                          (rec[i - 1 - lane] & kRecArrival) == uint32_t(j - 1 - lane);
-        const uint32_t hit = __ballot_sync(0xffffffffu, same);
-        const int q = hit ? __ffs(hit) : p;
-        if (lane < q) rec[i - lane] = (lane == 0 ? arrival : uint32_t(j - lane)) | kLeaveDiag;
-        if (hit) return {0u, 0, true};
-        i -= p;
-        j -= p;
-        arrival = uint32_t(j);
+        if (advance(p, 1, 0u, kLeaveDiag)) return {0u, 0, true};
         if (i == lo) break;
-        pl.set_row(i);
       } else if (hd == kDirStop) {
         if (lane == 0) rec[i] = arrival | kLeaveStop;
         return {kExitStop | (local ? 0u : kExitBad) | uint32_t(j), i, false};
@@ -415,19 +435,19 @@ __device__ __forceinline__ SegWalk walk_segment(Plane &pl, uint32_t *rec, int hi
       }
     } else {
       // E and F runs end inside the matrix; if the planes say otherwise, stop.
+      // The cells that extend the gap at once, the one that opened it by itself
+      // (128 x 20,000, one long gap: 3.79 ms a call cell by cell, 1.89 like this).
       if (j <= 0) return {kExitBad | kExitStop, i, false};
-      const int d = pl.nib(j);
+      (void)pl.nib(j);
+      const uint32_t gm = state == 1 ? pl.template gap_mask<true>(i, j) : pl.template gap_mask<false>(i, j);
+      const int p = gm == 0xffffffffu ? 32 : __ffs(~gm) - 1;
       if (state == 1) {
-        --j;
-        if (d & 4) state = 0;
+        j -= max(p, 1);
+        if (p == 0) state = 0;
       } else {
-        if (lane == 0) rec[i] = arrival | kLeaveUp;
-        --i;
-        if (d & 8) state = 0;
-        arrival = uint32_t(j) | uint32_t(state) << 20;
+        if (p == 0) state = 0;
+        if (advance(min(max(p, 1), i - lo), 0, uint32_t(state) << 20, kLeaveUp)) return {0u, 0, true};
         if (i == lo) break;
-        if (i >= floor && (rec[i] & kRecArrival) == arrival) return {0u, 0, true};
-        pl.up();
       }
     }
   }
