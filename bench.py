@@ -637,8 +637,8 @@ def configs_leg(c3_pairs=12):
     t0 = time.perf_counter()
     res = A.align_batch(ps, matrix="dna", gap_open=5, gap_extend=2, output="alignment")
     c3_s = time.perf_counter() - t0
-    # The same call with int32 lanes throughout (the int32 CTA fill for the
-    # long pairs); every result must equal the default run's.
+    # The same call with int32 lanes throughout (int32 strips for the long
+    # pairs); every result must equal the default run's.
     t0 = time.perf_counter()
     res32 = A.align_batch(ps, matrix="dna", gap_open=5, gap_extend=2, output="alignment", lane="i32")
     c3_i32_s = time.perf_counter() - t0
@@ -789,11 +789,10 @@ def traceback_uneven(O, A, W, cores, sample=2000):
 
 def long_pair_kernels(ps, per_sm=2):
     """Rooflines of the long-pair kernels: a device-resident batch of the
-    first long DNA pairs, per_sm of them per SM (one 16-warp CTA is resident
-    per SM; the second pair per SM evens out the first pairs' uneven
-    lengths) as far as their traceback planes fit in 40 % of the free HBM
-    (at most 120 GB): the strip traceback fill in int16x2 lanes, then one
-    walker warp per pair, timed by the batch's own events."""
+    first long DNA pairs, per_sm of them per SM (which evens out their
+    uneven lengths) as far as their traceback planes fit in 40 % of the free HBM
+    (at most 120 GB): the strip traceback fill in int16x2 lanes, then the
+    walk, timed by the batch's own events."""
     import torch
 
     from tweakseq_gb300 import aligner as A
@@ -835,7 +834,7 @@ def long_pair_kernels(ps, per_sm=2):
                          "note": f"{n_pairs} pairs in strips of 512 rows, one warp each"},
             "plane_writes": {"bound": "hbm", "achieved": plane_gbs, "peak": hbm, "unit": "GB/s",
                              "frac": plane_gbs / hbm, "bytes_per_cell": 0.5, "peak_source": hbm_src}},
-        "walk_warp_kernel": {
+        "walk_block_kernel": {
             "ms": walk_s * 1e3, "note": "device time after the fill: the walker and the result copies",
             "roofline": {"bound": "latency", "achieved": walk_bytes / walk_s / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": walk_bytes / walk_s / 1e9 / hbm, "bytes": walk_bytes,
@@ -938,7 +937,7 @@ def msa_leg(cpu_cols=40, cpu_tree_leaves=1000):
 
 def run_profile_case(args):
     """Small cases for ncu of the kernels behind the other measurements:
-    long_dna (32 DNA pairs of 10-12 kb with traceback: the CTA fill and the
+    long_dna (32 DNA pairs of 10-12 kb with traceback: the strip fill and the
     walker),
     identity (200,000 pairs of the guide-tree all-vs-all: the identity
     fill), traceback (20,000 of the uneven pairs with traceback: the

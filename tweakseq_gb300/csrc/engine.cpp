@@ -963,7 +963,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
         const PairDev &pd = b->pairs_h[size_t(k)];
         int8_t lt = 0;
         // A tuned table may prefer int32 over int16x2 for this length bucket,
-        // or the CTA fill for its int32 pairs.
+        // or the long pairs' fill for its int32 pairs.
         TunedChoice tc;
         const bool tuned = ch.use_table && !ch.force.shape && tune_table_pick(b->out_mode, pd.a_len, pd.b_len, &tc);
         if (try16 && !(tuned && tc.sh.i16 == 0)) {

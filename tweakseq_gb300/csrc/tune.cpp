@@ -7,14 +7,14 @@
 //   - the lane width G (4, 8, 16 or 32 lanes per pair);
 //   - for score output, the lane type: int16x2 (proven or overflow-checked
 //     with the exact int32 re-run) against int32;
-//   - for buckets of 1,024 residues and more, the CTA fill (one pair per
-//     8-warp CTA, the pair's bands striped over the warps) against one pair
+//   - for buckets of 1,024 residues and more, the long pairs' fill (strips,
+//     one pair over many warps; identity: a CTA of 8 warps) against one pair
 //     per warp group.
 // The table is written as JSON and read back by tsq_tune_load; batches
 // created with opts.autotune consult it.  Few-pair batches still get at
 // least enough lanes per pair to keep every SM busy (the planner takes the
 // larger of the tuned and the occupancy G), and a pair too long for any
-// warp group keeps the CTA fill whatever the table says.
+// warp group keeps the long pairs' fill whatever the table says.
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
@@ -32,7 +32,7 @@ namespace {
 struct Entry {
   int out, lo, hi;
   Shape sh;  // G, R, and i16 (1: int16x2 lanes where their range allows, 0: int32)
-  int cta;   // 1: int32 pairs of the bucket take the CTA fill
+  int cta;   // 1: int32 pairs of the bucket take the long pairs' fill
   double gcups;
 };
 
@@ -44,7 +44,7 @@ bool g_loaded = false;
 constexpr int kEdges[] = {0, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 3072, 4096, 6144, 8192, 1 << 21};
 constexpr int kNumBuckets = int(sizeof(kEdges) / sizeof(kEdges[0])) - 1;
 constexpr int kWidths[] = {4, 8, 16, 32};
-constexpr int kCtaFrom = 1024;  // buckets from this length also try the CTA fill
+constexpr int kCtaFrom = 1024;  // buckets from this length also try the long pairs' fill
 const char *kOutNames[] = {"score", "identity", "alignment"};
 
 int find_int(const std::string &obj, const char *key, int *v) {
@@ -170,7 +170,7 @@ extern "C" int tsq_tune_run(const char *json_path, int32_t quick) {
       p.gap_extend = 1;
       p.mode = TSQ_GLOBAL;
       p.output = out == kOutScore ? TSQ_OUT_SCORE : (out == kOutIdent ? TSQ_OUT_IDENTITY : TSQ_OUT_ALIGNMENT);
-      // Candidates: (lane width, lane type, CTA fill).  Each is timed as the
+      // Candidates: (lane width, lane type, long pairs' fill).  Each is timed as the
       // fill time of one planned run (device events), the best of several.
       // The first candidate is the planner's own choice (nothing forced);
       // a forced candidate replaces it only when it is at least 3 % faster,
