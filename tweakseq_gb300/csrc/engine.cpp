@@ -769,10 +769,7 @@ void plan_strips(tsq_batch *b, PlanScratch &ps, int64_t s, int64_t e, StripKind 
       list.push_back(make_int2(int32_t(q - s), st));
     }
     off.push_back(entries);
-    // The hand-over row; later the walk's records where those need the room.
-    int64_t room = strips > 1 ? pd.b_len : 0;
-    if (b->fill_mode == kOutTrace && pd.a_len >= kWalkRecRows) room = std::max<int64_t>(room, (pd.a_len + 2) / 2);
-    entries += (room + 15) & ~int64_t(15);
+    entries += strip_row_entries(pd.a_len, pd.b_len, rows, b->fill_mode == kOutTrace);
     L.max_rows = std::max(L.max_rows, pd.a_len);
   }
   for (SortRec &r : key) r.key = most - r.key;

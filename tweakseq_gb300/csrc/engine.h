@@ -270,6 +270,16 @@ int collect_one(const ResultDev &d, const char *rows, int64_t cap, tsq_result &o
 // Releases the rows of results that collect_one filled (those without are left).
 void free_rows(tsq_result *r, int64_t n);
 
+// The device block of the one-pair path: byte offsets of its parts, in order.
+struct PairLayout {
+  int64_t up_bytes;    // the upload block, at 0
+  int64_t codes, ccodes;
+  int64_t res, down_bytes;  // the result record, then the gapped rows: copied back
+  int64_t row, row_bytes;   // the strips' row (strip_row_entries), cleared before the fill
+  int64_t planes, total;
+};
+PairLayout pair_layout(int32_t la, int32_t lb, StripKind kind, int out_mode);
+
 // The plain form's one-pair path (pair.cpp).  One object per host thread.
 struct PairPath {
   int device = -1;

@@ -69,6 +69,22 @@ static_assert(sizeof(PairDev) <= kOffTask && sizeof(ResultDev) == 32, "record si
 
 }  // namespace
 
+PairLayout pair_layout(int32_t la, int32_t lb, StripKind kind, int out_mode) {
+  const bool walk = out_mode != kOutScore, emit = out_mode == kOutTrace;
+  const int64_t len = int64_t(la) + lb;
+  PairLayout l;
+  l.up_bytes = int64_t(kOffSeqs) + len + kPad;
+  l.codes = align256(l.up_bytes);
+  l.ccodes = l.codes + align256(len + kPad);
+  l.res = l.ccodes + align256(len + kPad);
+  l.down_bytes = int64_t(sizeof(ResultDev)) + (emit ? 2 * len : 0);
+  l.row = l.res + align256(l.down_bytes);
+  l.row_bytes = 8 * strip_row_entries(la, lb, strip_rows(kind), walk);
+  l.planes = l.row + align256(l.row_bytes);
+  l.total = l.planes + std::max<int64_t>(walk ? plane_bytes(la, lb, strip_shape(kind)) : 0, 16);
+  return l;
+}
+
 void PairPath::reset() {
   if (stream) cudaStreamSynchronize(stream);
   dev.release();
@@ -118,31 +134,20 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   const int blocks_avail = strip_blocks(kind, fill_mode, local, sc.nclasses);
   if (blocks_avail <= 0) return TSQ_E_CUDA;
 
-  // ---- device layout ---------------------------------------------------
+  // ---- device block ----------------------------------------------------
   const int64_t len = int64_t(la) + lb;
-  const int64_t up_bytes = int64_t(kOffSeqs) + len + kPad;
-  const int64_t off_codes = align256(up_bytes);
-  const int64_t off_ccodes = off_codes + align256(len + kPad);
-  const int64_t off_res = off_ccodes + align256(len + kPad);
-  const int64_t down_bytes = int64_t(sizeof(ResultDev)) + (emit ? 2 * len : 0);  // record, then a and b rows
-  const int64_t off_bnd = off_res + align256(down_bytes);
-  // The strips' hand-over row, later the walk's records where those need it.
-  int64_t bnd_bytes = n_units > 1 ? (int64_t(lb) + 15) / 16 * 16 * 8 : 0;
-  if (out_mode != kOutScore && la >= kWalkRecRows) bnd_bytes = std::max(bnd_bytes, (int64_t(la) + 3) / 4 * 16);
-  const int64_t off_planes = off_bnd + align256(bnd_bytes);
-  const int64_t plane_total = walk ? plane_bytes(la, lb, shp) : 0;
-  const int64_t dev_bytes = off_planes + std::max<int64_t>(plane_total, 16);
+  const PairLayout lay = pair_layout(la, lb, kind, out_mode);
 
   auto grow = [](size_t need, size_t cap) { return need <= cap ? need : need + need / 2; };
   // (A pair whose traceback planes do not fit in device memory fails here
   // with TSQ_E_NOMEM, as it does on the batch engine's one-pair plan.)
-  if (const cudaError_t e = pp->dev.ensure(grow(size_t(dev_bytes), pp->dev.cap), st); e != cudaSuccess) {
+  if (const cudaError_t e = pp->dev.ensure(grow(size_t(lay.total), pp->dev.cap), st); e != cudaSuccess) {
     if (e != cudaErrorMemoryAllocation || emit || !walk) return cuda_status(e);
     cudaGetLastError();
     return kPairNotTaken;
   }
-  PAIR_TRY(pp->up.ensure(grow(size_t(up_bytes), pp->up.cap)));
-  PAIR_TRY(pp->down.ensure(grow(size_t(down_bytes), pp->down.cap)));
+  PAIR_TRY(pp->up.ensure(grow(size_t(lay.up_bytes), pp->up.cap)));
+  PAIR_TRY(pp->down.ensure(grow(size_t(lay.down_bytes), pp->down.cap)));
 
   // ---- the upload block --------------------------------------------------
   uint8_t *h = pp->up.as<uint8_t>();
@@ -161,13 +166,13 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
 
   uint8_t *d = pp->dev.as<uint8_t>();
   const uint8_t *seqs = d + kOffSeqs;
-  uint8_t *codes = d + off_codes;
-  uint8_t *ccodes = d + off_ccodes;
-  ResultDev *res = reinterpret_cast<ResultDev *>(d + off_res);
-  PAIR_TRY(cudaMemcpyAsync(d, h, size_t(up_bytes), cudaMemcpyHostToDevice, st));
+  uint8_t *codes = d + lay.codes;
+  uint8_t *ccodes = d + lay.ccodes;
+  ResultDev *res = reinterpret_cast<ResultDev *>(d + lay.res);
+  PAIR_TRY(cudaMemcpyAsync(d, h, size_t(lay.up_bytes), cudaMemcpyHostToDevice, st));
   // (It also clears the hand-over row, and the launches after it start early: the
   // gaps between a short pair's launches are a tenth of its call.)
-  PAIR_TRY(launch_encode(seqs, len + kPad, d + kOffLut, codes, d + kOffClut, ccodes, st, d + off_bnd, bnd_bytes));
+  PAIR_TRY(launch_encode(seqs, len + kPad, d + kOffLut, codes, d + kOffClut, ccodes, st, d + lay.row, lay.row_bytes));
 
   // ---- fill ----------------------------------------------------------------
   FillArgs fa{};
@@ -181,19 +186,19 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   fa.gap_open = p->gap_open;
   fa.gap_extend = p->gap_extend;
   fa.res = res;
-  fa.planes = d + off_planes;
+  fa.planes = d + lay.planes;
   fa.plane_off = reinterpret_cast<const int64_t *>(d + kOffPlaneOff);
   fa.max_score = sc.max_score;
   fa.ccodes = ccodes;
   fa.cmatrix = reinterpret_cast<const int8_t *>(d + kOffCmatrix);
   fa.nclasses = sc.nclasses;
   fa.strip_ctl = reinterpret_cast<StripCtl *>(d + kOffCtl);
-  fa.strip_rows = reinterpret_cast<uint64_t *>(d + off_bnd);
+  fa.strip_rows = reinterpret_cast<uint64_t *>(d + lay.row);
   fa.strip_row_off = reinterpret_cast<const int64_t *>(d + kOffRowOff);
   PAIR_TRY(launch_strip(kind, fill_mode, local, fa, std::min(blocks_avail, n_units), st, true));
 
   // ---- traceback ---------------------------------------------------------
-  char *rows = reinterpret_cast<char *>(d + off_res + sizeof(ResultDev));
+  char *rows = reinterpret_cast<char *>(d + lay.res + sizeof(ResultDev));
   if (walk) {
     WalkArgs w{};
     w.seqs = seqs;
@@ -214,7 +219,7 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
     w.rec_off = fa.strip_row_off;
     PAIR_TRY(launch_walk_block(w, shp.R, la, st, true));
   }
-  PAIR_TRY(cudaMemcpyAsync(pp->down.p, res, size_t(down_bytes), cudaMemcpyDeviceToHost, st));
+  PAIR_TRY(cudaMemcpyAsync(pp->down.p, res, size_t(lay.down_bytes), cudaMemcpyDeviceToHost, st));
   PAIR_TRY(cudaStreamSynchronize(st));
 
   const ResultDev rd = *pp->down.as<ResultDev>();

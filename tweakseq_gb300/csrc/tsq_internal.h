@@ -17,6 +17,7 @@
 //              lanes of a group store one contiguous run per step.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <cstddef>
 
@@ -141,8 +142,8 @@ struct WalkArgs {
   char *aln;                 // per pair: 2 * cap bytes (a row then b row)
   const int64_t *aln_off;
   int32_t skip_begin, skip_end;  // launch_walk: tasks that another launch walks
-  // launch_walk_block: per task, (a_len + 2) / 2 entries for the path's records
-  // (used by pairs whose records do not fit shared memory).
+  // launch_walk_block: per task, the pair's row (strip_row_entries), for the
+  // path's records of pairs whose records do not fit shared memory.
   uint64_t *rec_rows;
   const int64_t *rec_off;
   int32_t rec_words;
@@ -221,6 +222,15 @@ cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st);
 // The pairs of a strip launch, one block each; max_rows: their longest a.
 // Pairs of at least kWalkRecRows rows need room for their records.
 constexpr int32_t kWalkRecRows = 32768;
+// 64-bit entries of a pair's row in global memory in strips of `rows` rows: its
+// n hand-over entries where there is more than one strip; walked pairs of
+// kWalkRecRows rows and more keep the walk's 32-bit records of rows 0 to m there
+// afterwards.  In whole 128 bytes.
+inline int64_t strip_row_entries(int32_t m, int32_t n, int rows, bool walk) {
+  int64_t entries = m > rows ? n : 0;
+  if (walk && m >= kWalkRecRows) entries = std::max<int64_t>(entries, (int64_t(m) + 2) / 2);
+  return (entries + 15) & ~int64_t(15);
+}
 cudaError_t launch_walk_block(const WalkArgs &a, int R, int32_t max_rows, cudaStream_t st, bool early = false);
 // Residues -> letter codes and, when clut_dev / ccodes are set, score
 // classes.
