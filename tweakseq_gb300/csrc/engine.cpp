@@ -628,9 +628,9 @@ int batch_plan_chunk(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, 
 }
 
 int input_segment(const tsq_batch *owner, const uint8_t *seqs, int64_t begin, int64_t end, cudaStream_t stream) {
-  if (!owner || begin < 0 || end > owner->seqs_len || begin % 16 != 0 || (end > begin && !seqs))
-    return TSQ_E_INVALID_ARG;
-  if (end <= begin) return TSQ_OK;
+  if (!owner || begin < 0 || end > owner->seqs_len) return TSQ_E_INVALID_ARG;
+  if (end <= begin) return TSQ_OK;  // (earlier segments may end with the buffer, at any byte)
+  if (begin % 16 != 0 || !seqs) return TSQ_E_INVALID_ARG;
   TSQ_TRY(cudaMemcpyAsync(owner->seqs.as<uint8_t>() + begin, seqs + begin, size_t(end - begin),
                           cudaMemcpyHostToDevice, stream));
   TSQ_TRY(launch_encode(owner->seqs.as<uint8_t>() + begin, end - begin, owner->lut.as<uint8_t>(),
