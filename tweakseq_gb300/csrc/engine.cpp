@@ -727,18 +727,6 @@ int prepare_object(tsq_batch *b, const tsq_params *p, const tsq_batch_opts *opts
 // more, a warp for each pair fills the GPU and walks no cell twice.
 constexpr int32_t kManyWalks = 1024;
 
-// A pair is long when its sweep on one 32-lane group takes more steps than
-// kLongSteps and kLongShare of the batch's balanced per-lane work.  Device
-// time of protein batches (log-normal lengths, median as named), shares of
-// 0.5 / 1 / 2 / 4 and no strips: 1,000 x 800 score 0.93 / 0.89 / 0.69 / 0.66 and
-// 1.53 ms, with traceback 1.91 / 1.82 / 1.57 / 1.59 and 3.27; 10,000 x 350 score
-// 0.77 / 0.77 / 0.81 / 1.16 and 1.38: below 1 short pairs pay for strips they
-// do not fill, above 2 the longest pairs on one warp are the tail.  A lone
-// warp is as fast as strips up to about 600 steps (20 pairs x 150: 0.067 ms
-// either way).  Identity output's long form is a CTA of 8 warps, worth its
-// int32 cells from 20,000 steps.
-constexpr double kLongSteps = 600.0, kLongShare = 1.5, kLongStepsCta = 20000.0;
-
 // The strip launch of the pairs at [s, e) of the sorted order: its units,
 // most work left below first (a pair's strips stay in order), the pairs'
 // records and hand-over rows.
@@ -951,7 +939,8 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
     const double lanes = double(sms) * 24.0 * 32.0;
     const bool strips = b->fill_mode != kOutIdent;
     const double balanced = plain ? 0.0 : double(shape_cells) / (lanes * kR);
-    const double long_steps = strips ? std::max(kLongSteps, kLongShare * balanced) : std::max(kLongStepsCta, balanced);
+    const double long_steps =
+        strips ? strip_long_steps(plain ? 0.0 : double(shape_cells), sms) : std::max(kLongStepsCta, balanced);
     const bool try16 = lanes16_possible(b->fill_mode, b->local, p->lane);
     const bool strip16 = strips && p->lane == TSQ_LANE_AUTO && strip16_supported(sc, p->gap_open, p->gap_extend);
     parallel_for(n, [&](int64_t lo, int64_t hi, int slot) {
@@ -968,14 +957,11 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
           if (r16.lower) lt = (r16.upper && p->lane == TSQ_LANE_AUTO) ? 1 : 2;
         }
         if (lt == 0 && pd.a_len > 0 && pd.b_len > 0) {
-          const double steps32 = double((pd.a_len + 255) / 256) * double(pd.b_len + 31);
-          if (steps32 > long_steps || ch.force.cta || (tuned && tc.cta)) lt = strip16 ? 4 : 3;
+          if (sweep_steps32(pd.a_len, pd.b_len) > long_steps || ch.force.cta || (tuned && tc.cta)) lt = strip16 ? 4 : 3;
         } else if (lt != 0 && strip16 && !ch.force.shape) {
-          // An int16x2 pair whose sweep on one 32-lane group -- ceil(m/512)
-          // passes of n+63 steps -- would be the batch's tail (and, when
+          // An int16x2 pair that would be the batch's tail (and, when
           // checked, might need an int32 re-run on one warp as well).
-          const double steps16 = double((pd.a_len + 511) / 512) * double(pd.b_len + 63);
-          if (steps16 > long_steps) lt = 4;
+          if (sweep_steps16(pd.a_len, pd.b_len) > long_steps) lt = 4;
         }
         lsel[size_t(k)] = lt;
         sp.n_checked += lt == 2;

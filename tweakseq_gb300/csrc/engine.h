@@ -247,6 +247,26 @@ int64_t cost_order(const tsq_pair_desc *pairs, int64_t n, std::vector<uint8_t> &
 // ---- per-pair rules shared by the planner and the one-pair path ----------
 // Rows per lane of every fill.
 constexpr int kFillRows = 8;
+// A pair is long when its sweep on one 32-lane group takes more steps than
+// kLongSteps and kLongShare of the batch's balanced per-lane work.  Device
+// time of protein batches (log-normal lengths, median as named), shares of
+// 0.5 / 1 / 2 / 4 and no strips: 1,000 x 800 score 0.93 / 0.89 / 0.69 / 0.66 and
+// 1.53 ms, with traceback 1.91 / 1.82 / 1.57 / 1.59 and 3.27; 10,000 x 350 score
+// 0.77 / 0.77 / 0.81 / 1.16 and 1.38: below 1 short pairs pay for strips they
+// do not fill, above 2 the longest pairs on one warp are the tail.  A lone
+// warp is as fast as strips up to about 600 steps (20 pairs x 150: 0.067 ms
+// either way).  Identity output's long form is a CTA of 8 warps, worth its
+// int32 cells from 20,000 steps.
+constexpr double kLongSteps = 600.0, kLongShare = 1.5, kLongStepsCta = 20000.0;
+// The steps of that sweep: ceil(m/256) bands of n+31 in int32, ceil(m/512) passes
+// of n+63 in int16x2.
+inline double sweep_steps32(int64_t m, int64_t n) { return double((m + 255) / 256) * double(n + 31); }
+inline double sweep_steps16(int64_t m, int64_t n) { return double((m + 511) / 512) * double(n + 63); }
+// The steps from which a score or alignment batch of so many cells takes a pair for
+// long.
+inline double strip_long_steps(double cells, int sms) {
+  return std::max(kLongSteps, kLongShare * cells / (double(sms) * 24.0 * 32.0 * kFillRows));
+}
 int out_mode_of(const tsq_params *p);
 bool lanes16_possible(int out_mode, bool local, int lane);
 bool classes_needed(int out_mode, bool local, int lane);

@@ -39,6 +39,8 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+constexpr int kWarpsPerSm = 16;  // most warps any fill kernel keeps resident per SM
+
 struct Request {
   uint64_t id = 0;
   tsq_params params{};
@@ -47,7 +49,8 @@ struct Request {
   std::vector<uint8_t> seqs;
   std::vector<tsq_pair_desc> pairs;
   int64_t cells = 0;
-  int64_t bytes = 0;      // device bytes without the boundary rows
+  int64_t bytes = 0;      // device bytes without the boundary and strip rows
+  int64_t strip_bytes = 0;  // rows of the pairs that may go to a strip launch, each at most a warp's boundary rows
   int32_t max_n = 0;
   Clock::time_point t_submit, t_done;
   enum State { kPending, kRunning, kDone, kCancelled } state = kPending;
@@ -123,12 +126,17 @@ struct tsq_server {
   int64_t r_outstanding_pairs = 0;
   int tend_resident();                               // called with the lock held
 
-  // Boundary rows a tick of npairs pairs needs for sequences up to max_n
-  // columns: 8 group rows per warp of the launch (no more warps than pairs,
-  // no more than fit on the device), at the largest entry size (16 bytes).
-  int64_t boundary_bytes(int32_t max_n, int64_t npairs) const {
-    const int64_t warps = std::min<int64_t>(resident_warps, npairs + 8);
-    return warps * 8 * (int64_t(max_n) + 64) * 16;
+  // Boundary rows of one warp for sequences up to n columns: eight groups' rows
+  // at the largest entry size (16 bytes).
+  static int64_t warp_rows_bytes(int32_t n) { return 8 * (int64_t(n) + 64) * 16; }
+  // Boundary and strip rows a tick of npairs pairs needs for sequences up to
+  // max_n columns: a warp's rows for every warp of the launch (no more warps than
+  // pairs, no more than fit on the device).  A pair in strips has a row of its own
+  // and leaves its warp's to others, so strip rows count for the pairs beyond the
+  // warps alone.
+  int64_t row_bytes(int32_t max_n, int64_t npairs, int64_t strip_bytes) const {
+    const int64_t warps = std::min<int64_t>(resident_warps, npairs + 8), per_warp = warp_rows_bytes(max_n);
+    return warps * per_warp + std::min(strip_bytes, (npairs + 8 - warps) * per_warp);
   }
 
   void run();
@@ -319,7 +327,7 @@ void tsq_server::run() {
       const std::shared_ptr<Request> head = pending.front();
       const int64_t room = opts.hbm_budget_bytes - reserved;
       std::vector<std::shared_ptr<Request>> take;
-      int64_t bytes = 0, cells = 0, npairs = 0;
+      int64_t bytes = 0, strip_bytes = 0, cells = 0, npairs = 0;
       int32_t max_n = 0;
       for (auto it = pending.begin(); it != pending.end();) {
         const auto &r = *it;
@@ -329,7 +337,7 @@ void tsq_server::run() {
         }
         const int32_t mn = std::max(max_n, r->max_n);
         const int64_t np = npairs + int64_t(r->pairs.size());
-        const int64_t need = bytes + r->bytes + boundary_bytes(mn, np);
+        const int64_t need = bytes + r->bytes + row_bytes(mn, np, strip_bytes + r->strip_bytes);
         const bool first = take.empty();
         if (need > room || (!first && cells + r->cells > opts.max_tick_cells)) {
           if (first) ++admission_waits;
@@ -337,6 +345,7 @@ void tsq_server::run() {
         }
         take.push_back(r);
         bytes += r->bytes;
+        strip_bytes += r->strip_bytes;
         cells += r->cells;
         npairs = np;
         max_n = mn;
@@ -344,7 +353,7 @@ void tsq_server::run() {
         it = pending.erase(it);
       }
       if (!take.empty()) {
-        const int64_t tick_bytes = bytes + boundary_bytes(max_n, npairs);
+        const int64_t tick_bytes = bytes + row_bytes(max_n, npairs, strip_bytes);
         reserved += tick_bytes;
         peak_reserved = std::max(peak_reserved, reserved);
         ++ticks;
@@ -394,7 +403,7 @@ int tsq_server_create(const tsq_server_opts *opts, tsq_server **out) {
     }
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return TSQ_E_CUDA;
-    s->resident_warps = sms * 16;  // most warps any fill kernel keeps resident per SM
+    s->resident_warps = sms * kWarpsPerSm;
     if (s->opts.resident) {
       // The loop's arena comes out of the budget: a quarter of it, at most
       // 4 GiB.
@@ -441,15 +450,28 @@ int tsq_server_submit(tsq_server *s, const uint8_t *seqs, int64_t seqs_len, cons
         return TSQ_E_INVALID_ARG;
       r->cells += int64_t(d.a_len) * d.b_len;
       r->max_n = std::max(r->max_n, d.b_len);
-      bytes += 8 * std::max<int64_t>(d.b_len, d.a_len / 2) + 64;  // a long pair's hand-over row (or walk records) and record
       if (p->output == TSQ_OUT_ALIGNMENT)
         bytes += tsq::plane_bytes(d.a_len, d.b_len, tsq::Shape{32, 8, 0}) + 2 * (int64_t(d.a_len) + d.b_len);
+    }
+    // Pairs that may go to a strip launch: the more cells a tick has, the longer
+    // those are (a tuned table can send any).  Identity requests have none.
+    const int sms = s->resident_warps / kWarpsPerSm, rows = tsq::strip_rows(tsq::kStrip32);
+    const double long_steps = s->opts.autotune ? 0.0 : tsq::strip_long_steps(double(r->cells), sms);
+    for (const tsq_pair_desc &d : r->pairs) {
+      if (p->output == TSQ_OUT_IDENTITY || std::max(tsq::sweep_steps32(d.a_len, d.b_len),
+                                                    tsq::sweep_steps16(d.a_len, d.b_len)) <= long_steps)
+        continue;
+      const int64_t need = 8 * tsq::strip_row_entries(d.a_len, d.b_len, rows, p->output == TSQ_OUT_ALIGNMENT) +
+                           int64_t(sizeof(tsq::StripCtl)) + 8 * (1 + int64_t(d.a_len) / rows + 1);
+      const int64_t share = std::min(need, tsq_server::warp_rows_bytes(d.b_len));
+      r->strip_bytes += share;
+      bytes += need - share;
     }
     r->bytes = bytes;
     r->resident = s->loop && tsq::resident::Loop::eligible(r->params, r->pairs);
     std::lock_guard<std::mutex> lock(s->mu);
     if (s->stop) return TSQ_E_CANCELLED;
-    if (!r->resident && r->bytes + s->boundary_bytes(r->max_n, n) > s->opts.hbm_budget_bytes) {
+    if (!r->resident && r->bytes + s->row_bytes(r->max_n, n, r->strip_bytes) > s->opts.hbm_budget_bytes) {
       ++s->rejected;
       return TSQ_E_REJECTED;
     }
