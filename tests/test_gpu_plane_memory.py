@@ -1,0 +1,82 @@
+"""Device memory of identity calls: traceback planes are a workspace that gives
+way -- to a call's own second try, to alignment calls of the same thread, and to
+what others have left free."""
+import threading
+
+import numpy as np
+import pytest
+
+from tweakseq_gb300 import aligner as A
+from tweakseq_gb300 import build as B
+
+pytestmark = pytest.mark.gpu
+GB = 1 << 30
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    B.build()
+
+
+def on_own_thread(f):
+    """Runs f on a thread of its own: the library's cached engines are the
+    thread's, and go with it."""
+    out = {}
+
+    def run():
+        try:
+            out["value"] = f()
+        except BaseException as e:  # noqa: BLE001 (handed to the caller)
+            out["error"] = e
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    if "error" in out:
+        raise out["error"]
+    return out.get("value")
+
+
+def free_bytes():
+    import torch
+
+    return torch.cuda.mem_get_info()[0]
+
+
+def leave_free(keep):
+    """A buffer that leaves `keep` bytes of device memory free."""
+    import torch
+
+    torch.cuda.empty_cache()
+    return torch.empty(free_bytes() - keep, dtype=torch.uint8, device="cuda")
+
+
+def equal_pairs(n, length):
+    """n pairs of `length` residues out of one buffer, at shifting offsets."""
+    rng = np.random.default_rng(length)
+    seqs = np.frombuffer(b"ARNDCQEGHILKMFPSTWYV", dtype=np.uint8)[rng.integers(0, 20, length + 4096)]
+    k = np.arange(n)
+    return seqs, (k * 7) % 4096, np.full(n, length), (k * 7 + 3) % 4096, np.full(n, length)
+
+
+def identity(pairs):
+    return A.align_batch(pairs, output="identity").table
+
+
+def test_second_try_releases_the_planes_of_the_first(monkeypatch):
+    torch = pytest.importorskip("torch")
+    pairs = equal_pairs(32768, 740)  # two chunks, 4.2 and 8.4 GB of planes
+
+    def body():
+        monkeypatch.setenv("TSQ_WAVE_BUDGET_BYTES", "1")
+        want = identity(pairs)
+        monkeypatch.delenv("TSQ_WAVE_BUDGET_BYTES")
+        hold = leave_free(6 * GB)
+        got = identity(pairs)
+        left = free_bytes()
+        del hold
+        torch.cuda.empty_cache()
+        assert np.array_equal(got, want)
+        assert left > 4.5 * GB, left / GB
+
+    on_own_thread(body)

@@ -66,6 +66,11 @@ int guarded(F &&f) {
   }
 }
 
+// The planes of an earlier identity call's later chunks (nothing of it runs any more).
+void release_chunk_planes(ThreadCache &c) {
+  for (const std::unique_ptr<tsq_batch> &x : c.chunk_engines) x->planes.release();
+}
+
 // A large score or identity call runs as a few chunks, each planned by its
 // own batch object and run on its own stream; each later chunk is planned on
 // the host while the earlier ones run, and the chunks' persistent launches
@@ -373,6 +378,10 @@ int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *
       const int rc = align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, planes);
       if (rc != TSQ_E_NOMEM || !planes) return rc;
       cudaGetLastError();
+      // The planes that some chunks did get go back first.
+      e->planes.release();
+      release_chunk_planes(c);
+      tsq::trim_engine_pool(dev);
       return align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, false);
     }
     int rc = tsq::batch_plan(e, seqs, seqs_len, pairs, n, p, opts, false);
