@@ -80,3 +80,24 @@ def test_second_try_releases_the_planes_of_the_first(monkeypatch):
         assert left > 4.5 * GB, left / GB
 
     on_own_thread(body)
+
+
+def test_alignments_take_back_an_identity_calls_planes():
+    torch = pytest.importorskip("torch")
+    pairs = equal_pairs(32768, 500)  # 2.2 GB of planes in one chunk's engine, 4.4 in the other's
+    rng = np.random.default_rng(5)
+    a = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(0, 4, 92_000)]
+    two = (a, [0, 0], [len(a)] * 2, [0, 0], [len(a)] * 2)  # 4.2 GB of planes each
+
+    def body():
+        identity(pairs)
+        hold = leave_free(3 * GB)
+        try:
+            got = A.align_batch(two, matrix="dna", gap_open=5, gap_extend=2, output="alignment")
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        assert got.table["score"].tolist() == [2 * len(a)] * 2
+        assert got.aln_a[0] == got.aln_b[1] == a.tobytes().decode()
+
+    on_own_thread(body)

@@ -365,9 +365,10 @@ int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *
       int64_t budget = 0;
       if (!wave_budget(&budget)) return TSQ_E_CUDA;
       if (total > budget) {
-        // Memory the engine's pool keeps mapped but does not use goes back
-        // first (only when the batch would not fit: unmapping costs about as
-        // much as mapping).
+        // Memory the engine's pool keeps mapped but does not use, and the
+        // planes of an identity call's chunks, go back first (only when the
+        // batch would not fit: unmapping costs about as much as mapping).
+        release_chunk_planes(c);
         tsq::trim_engine_pool(dev);
         if (!wave_budget(&budget)) return TSQ_E_CUDA;
       }
