@@ -101,3 +101,35 @@ def test_alignments_take_back_an_identity_calls_planes():
         assert got.aln_a[0] == got.aln_b[1] == a.tobytes().decode()
 
     on_own_thread(body)
+
+
+@pytest.mark.parametrize("form", ["one of a batch", "pair", "resident"])
+def test_other_calls_take_back_an_identity_calls_planes(form):
+    """4.2 GB of planes with 1.2 GB free and 6.6 GB in the identity call's engines."""
+    torch = pytest.importorskip("torch")
+    pairs = equal_pairs(32768, 500)
+    rng = np.random.default_rng(6)
+    a = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(0, 4, 92_000)]
+    kw = dict(matrix="dna", gap_open=5, gap_extend=2, output="alignment")
+
+    def align():
+        if form == "pair":
+            return A.align_pair(a.tobytes(), a.tobytes(), **kw)
+        one = (a, [0], [len(a)], [0], [len(a)])
+        if form == "one of a batch":
+            return A.align_batch(one, **kw)[0]
+        with A.Batch(one, use_graph=False, **kw) as b:
+            b.run()
+            return b.results()[0]
+
+    def body():
+        identity(pairs)
+        hold = leave_free(int(1.2 * GB))
+        try:
+            got = align()
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        assert got.score == 2 * len(a) and got.aln_a == got.aln_b == a.tobytes().decode()
+
+    on_own_thread(body)

@@ -67,8 +67,35 @@ int guarded(F &&f) {
 }
 
 // The planes of an earlier identity call's later chunks (nothing of it runs any more).
-void release_chunk_planes(ThreadCache &c) {
-  for (const std::unique_ptr<tsq_batch> &x : c.chunk_engines) x->planes.release();
+size_t release_chunk_planes(ThreadCache &c) {
+  size_t held = 0;
+  for (const std::unique_ptr<tsq_batch> &x : c.chunk_engines) {
+    held += x->planes.cap;
+    x->planes.release();
+  }
+  return held;
+}
+
+// Releases the planes that earlier calls left in the thread's cached engines; false
+// when there were none.
+bool release_idle_planes(ThreadCache &c) {
+  size_t held = release_chunk_planes(c);
+  for (tsq_batch *x : {c.batch_engine.get(), c.pair_engine.get()}) {
+    if (!x) continue;
+    held += x->planes.cap;
+    x->planes.release();
+  }
+  return held > 0;
+}
+
+// Runs f, which plans a call.  Without memory for it, once more without the planes
+// of earlier calls.
+template <class F>
+int with_idle_planes_back(ThreadCache &c, F &&f) {
+  const int rc = f();
+  if (rc != TSQ_E_NOMEM || !release_idle_planes(c)) return rc;
+  cudaGetLastError();
+  return f();
 }
 
 // A large score or identity call runs as a few chunks, each planned by its
@@ -296,7 +323,8 @@ int tsq_align_pair(const uint8_t *a, int32_t la, const uint8_t *b, int32_t lb, c
     if (!out || !p || la < 0 || lb < 0 || (la > 0 && !a) || (lb > 0 && !b)) return TSQ_E_INVALID_ARG;
     std::memset(out, 0, sizeof(*out));
     ThreadCache &c = cache();
-    const int lean = tsq::pair_align(&c.pair_path, a, la, b, lb, p, out);
+    const int lean =
+        with_idle_planes_back(c, [&] { return tsq::pair_align(&c.pair_path, a, la, b, lb, p, out); });
     if (lean != tsq::kPairNotTaken) return lean;
     // Calls the one-pair path leaves to the batch engine (forced checked
     // int16x2 lanes, pairs beyond its limits, bad parameters).
@@ -312,7 +340,8 @@ int tsq_align_pair(const uint8_t *a, int32_t la, const uint8_t *b, int32_t lb, c
     if (lb) std::memcpy(buf.get() + la, b, size_t(lb));
     tsq_pair_desc d{0, la, la, lb};
     tsq_batch *e = c.pair_engine.get();
-    int rc = tsq::batch_plan(e, buf.get(), int64_t(la) + lb, &d, 1, p, nullptr, true);
+    int rc = with_idle_planes_back(
+        c, [&] { return tsq::batch_plan(e, buf.get(), int64_t(la) + lb, &d, 1, p, nullptr, true); });
     if (rc) return rc;
     if ((rc = tsq::batch_run_async(e))) return rc;
     if ((rc = tsq::batch_sync(e))) return rc;
@@ -377,15 +406,15 @@ int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *
     if (p && p->output != TSQ_OUT_ALIGNMENT && n >= 2 * kChunkPairs && pairs) {
       const bool planes = tsq::identity_planes_fit(p, pairs, n);
       const int rc = align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, planes);
-      if (rc != TSQ_E_NOMEM || !planes) return rc;
+      // Without memory, once more without planes; those that earlier calls and
+      // some of the chunks did get go back first.
+      if (rc != TSQ_E_NOMEM || !(release_idle_planes(c) || planes)) return rc;
       cudaGetLastError();
-      // The planes that some chunks did get go back first.
-      e->planes.release();
-      release_chunk_planes(c);
       tsq::trim_engine_pool(dev);
       return align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, false);
     }
-    int rc = tsq::batch_plan(e, seqs, seqs_len, pairs, n, p, opts, false);
+    int rc = with_idle_planes_back(
+        c, [&] { return tsq::batch_plan(e, seqs, seqs_len, pairs, n, p, opts, false); });
     if (rc) return rc;
     if ((rc = tsq::batch_run_async(e))) return rc;
     if ((rc = tsq::batch_sync(e))) return rc;
@@ -399,7 +428,8 @@ int tsq_batch_create(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc 
     if (!out) return TSQ_E_INVALID_ARG;
     *out = nullptr;
     std::unique_ptr<tsq_batch> b(new tsq_batch());
-    const int rc = tsq::batch_plan(b.get(), seqs, seqs_len, pairs, n, p, opts, false);
+    const int rc = with_idle_planes_back(
+        cache(), [&] { return tsq::batch_plan(b.get(), seqs, seqs_len, pairs, n, p, opts, false); });
     if (rc) return rc;
     *out = b.release();
     return TSQ_OK;

@@ -141,7 +141,12 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
   auto grow = [](size_t need, size_t cap) { return need <= cap ? need : need + need / 2; };
   // (A pair whose traceback planes do not fit in device memory fails here
   // with TSQ_E_NOMEM, as it does on the batch engine's one-pair plan.)
-  if (const cudaError_t e = pp->dev.ensure(grow(size_t(lay.total), pp->dev.cap), st); e != cudaSuccess) {
+  cudaError_t e = pp->dev.ensure(grow(size_t(lay.total), pp->dev.cap), st);
+  if (e == cudaErrorMemoryAllocation) {  // (without room to grow)
+    cudaGetLastError();
+    e = pp->dev.ensure(size_t(lay.total), st);
+  }
+  if (e != cudaSuccess) {
     if (e != cudaErrorMemoryAllocation || emit || !walk) return cuda_status(e);
     cudaGetLastError();
     return kPairNotTaken;
@@ -224,8 +229,8 @@ int pair_align(PairPath *pp, const uint8_t *a, int32_t la, const uint8_t *b, int
 
   const ResultDev rd = *pp->down.as<ResultDev>();
   const char *hrows = pp->down.as<char>() + sizeof(ResultDev);
-  const int e = collect_one(rd, emit && rd.status == TSQ_OK ? hrows : nullptr, len, *out);
-  if (e) return e;
+  const int rc = collect_one(rd, emit && rd.status == TSQ_OK ? hrows : nullptr, len, *out);
+  if (rc) return rc;
   return rd.status;
 }
 
