@@ -133,3 +133,29 @@ def test_other_calls_take_back_an_identity_calls_planes(form):
         assert got.score == 2 * len(a) and got.aln_a == got.aln_b == a.tobytes().decode()
 
     on_own_thread(body)
+
+
+@pytest.mark.parametrize("resident", [False, True])
+def test_planes_take_a_share_of_what_is_free(resident, monkeypatch):
+    torch = pytest.importorskip("torch")
+    pairs = equal_pairs(32768, 500)  # 6.6 GB of planes
+
+    def run():
+        if not resident:
+            return identity(pairs), free_bytes()
+        with A.Batch(pairs, output="identity") as b:
+            b.run()
+            return b.results().table, free_bytes()
+
+    def body():
+        monkeypatch.setenv("TSQ_WAVE_BUDGET_BYTES", "1")
+        want, _ = run()
+        monkeypatch.delenv("TSQ_WAVE_BUDGET_BYTES")
+        hold = leave_free(8 * GB)
+        got, left = run()
+        del hold
+        torch.cuda.empty_cache()
+        assert np.array_equal(got, want)
+        assert left > 5 * GB, left / GB
+
+    on_own_thread(body)

@@ -404,7 +404,9 @@ int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len, const tsq_pair_desc *
       if (total > budget) return align_in_waves(e, seqs, seqs_len, pairs, n, p, opts, out, bytes, budget);
     }
     if (p && p->output != TSQ_OUT_ALIGNMENT && n >= 2 * kChunkPairs && pairs) {
-      const bool planes = tsq::identity_planes_fit(p, pairs, n);
+      int64_t held = int64_t(e->planes.cap);
+      for (const std::unique_ptr<tsq_batch> &x : c.chunk_engines) held += int64_t(x->planes.cap);
+      const bool planes = tsq::identity_planes_fit(p, pairs, n, dev, held);
       const int rc = align_in_chunks(c, e, seqs, seqs_len, pairs, n, p, opts, out, planes);
       // Without memory, once more without planes; those that earlier calls and
       // some of the chunks did get go back first.

@@ -443,10 +443,14 @@ int out_mode_of(const tsq_params *p) {
 // them without writing rows.  (123,753 protein pairs of 250-600 residues and
 // their 498-leaf tree: 25.7 against 17.8 ms.)
 // Larger batches, and server slots (whose admission does not count planes for
-// identity), carry the counts.
+// identity), carry the counts.  So do batches whose planes would take more than a
+// quarter of the memory that is free: they stay with the batch object or the
+// thread's engines, and other allocations of the process share the device.
 constexpr int64_t kIdentityPlaneBytes = int64_t(24) << 30;
+// (Below this the free memory is not looked up, 10 us a call.)
+constexpr int64_t kIdentityPlanesSmall = int64_t(256) << 20;
 
-bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n) {
+bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n, int device, int64_t held) {
   if (!p || p->output != TSQ_OUT_IDENTITY || n <= 0 || !pairs) return false;
   int64_t budget = kIdentityPlaneBytes;
   // (TSQ_WAVE_BUDGET_BYTES lowers it; tests use it to take the other way.)
@@ -463,7 +467,14 @@ bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_
   });
   int64_t total = 0;
   for (int64_t x : part) total += std::min(x, budget + 1);
-  return total <= budget;
+  if (total > budget) return false;
+  if (total <= std::max(kIdentityPlanesSmall, held)) return true;
+  size_t free_b = 0, total_b = 0;
+  if ((device >= 0 && cudaSetDevice(device) != cudaSuccess) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();  // (planning reports it)
+    return false;
+  }
+  return total <= (int64_t(free_b) + held) / 4;
 }
 
 int check_params(const tsq_params *p) {
@@ -607,7 +618,8 @@ int batch_plan(tsq_batch *b, const uint8_t *seqs, int64_t seqs_len, const tsq_pa
                const tsq_params *p, const tsq_batch_opts *opts, bool plain) {
   TraceRange tr(plain ? "plan (one pair)" : "plan");
   if (!b) return TSQ_E_INVALID_ARG;
-  b->identity_planes = b->identity_planes_allowed && identity_planes_fit(p, pairs, n);
+  b->identity_planes = b->identity_planes_allowed &&
+                       identity_planes_fit(p, pairs, n, opts ? opts->device : -1, int64_t(b->planes.cap));
   const int rc = plan_impl(b, nullptr, seqs, seqs_len, pairs, n, p, opts, plain, 0, 0, false);
   if (rc != TSQ_E_NOMEM || !b->identity_planes) return rc;
   cudaGetLastError();

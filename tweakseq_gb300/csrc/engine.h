@@ -270,8 +270,9 @@ inline double strip_long_steps(double cells, int sms) {
 int out_mode_of(const tsq_params *p);
 bool lanes16_possible(int out_mode, bool local, int lane);
 bool classes_needed(int out_mode, bool local, int lane);
-// Whether identity output of these pairs runs on traceback planes.
-bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n);
+// Whether identity output of these pairs runs on traceback planes.  device: -1 for the
+// current one; held: bytes of planes that the call's engines have already.
+bool identity_planes_fit(const tsq_params *p, const tsq_pair_desc *pairs, int64_t n, int device, int64_t held);
 // TSQ_E_INVALID_ARG for gap costs, mode, output or lane out of range.
 int check_params(const tsq_params *p);
 // TSQ_E_TOO_LARGE for a pair beyond the kernels' value and length ranges.
