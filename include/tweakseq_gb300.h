@@ -117,8 +117,10 @@ typedef struct {
   int32_t autotune;     /* 1 = consult the tuned table (tsq_tune_load) */
   int32_t wait_polls;   /* polls a bounded device-side wait makes before it
                            gives up and its pair reports TSQ_E_TIMEOUT (the
-                           long-pair fill's warps wait on one another);
-                           0 = the default, 4,194,304 */
+                           long-pair fill's warps wait on one another; a
+                           warp whose turn is far off sleeps up to 33 us
+                           between two polls); 0 = the default, 4,194,304,
+                           of which a sleep counts for 256 ns each */
 } tsq_batch_opts;
 
 /* Counters of the last run of a batch. */
