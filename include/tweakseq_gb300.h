@@ -119,8 +119,8 @@ typedef struct {
                            gives up and its pair reports TSQ_E_TIMEOUT (the
                            long-pair fill's warps wait on one another; a
                            warp whose turn is far off sleeps up to 33 us
-                           between two polls); 0 = the default, 4,194,304,
-                           of which a sleep counts for 256 ns each */
+                           between two polls); 0 = the default, 1,048,576,
+                           or 4,194,304 where the warps share a CTA */
 } tsq_batch_opts;
 
 /* Counters of the last run of a batch. */

@@ -43,6 +43,10 @@
 namespace tsq {
 namespace fill {
 
+// Polls of a wait by default: about 0.7 s for the strip above, 35 s where a strip's
+// turn is far off and it sleeps between them.
+constexpr int kStripPolls = 1 << 20;
+
 constexpr uint32_t kTagMask = 0x3FFFu;  // tags 1..16383
 static_assert((kMaxPairLen + 127) / 128 - 1 <= int64_t(kTagMask), "a tag for every strip that hands down");
 
@@ -79,13 +83,9 @@ template <int COLS>
 struct StripReader {
   const uint64_t *row;
   uint32_t tag;   // the tag of the strip above
-  int n, lane, limit, sleep_polls;
-  bool gave_up = false;
-  uint64_t ahead = 0u;
-  // spin_limit: FillArgs::spin_limit.
-  __device__ StripReader(const uint64_t *row, uint32_t tag, int n, int lane, int spin_limit)
-      : row(row), tag(tag), n(n), lane(lane), limit(spin_limit > 0 ? spin_limit : kSpinLimit),
-        sleep_polls(spin_limit > 0 ? 0 : 1) {}
+  int n, lane, limit;
+  bool gave_up;
+  uint64_t ahead;
   __device__ uint64_t fetch(int chunk) const {
     const int col = COLS * chunk + lane;
     return lane < COLS && col < n ? strip_load(row + col) : uint64_t(tag);
@@ -103,12 +103,10 @@ struct StripReader {
       // All strips of a pair wait on the same few entries at first: each
       // sleeps about as long as the strips between take to get there (40
       // steps of some 50 ns each), or thousands of polls of one address would
-      // hold the writer up.  Under the default limit a sleep counts as the polls
-      // it stands for, so that a wait ends within seconds; a caller's limit counts
-      // polls.
+      // hold the writer up.
       const uint32_t away = tag - __shfl_sync(0xffffffffu, uint32_t(v) & kTagMask, 0);
       const uint32_t ns = away <= 1u ? 0u : min(away, 64u) * 512u;
-      polls += 1 + sleep_polls * int(ns / 256u);
+      ++polls;
       if (ns) __nanosleep(ns);
       v = fetch(chunk);
     }

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
       uint64_t *row = A.strip_rows + A.strip_row_off[q];
       const uint32_t tag = strip_tag(strip);
       const bool hands_down = strip + 1 < strips;
-      StripReader<C> rd(row, strip_tag(strip - 1), n, t, A.spin_limit);
+      StripReader<C> rd{row, strip_tag(strip - 1), n, t, A.spin_limit > 0 ? A.spin_limit : kStripPolls, false, 0u};
       if (strip > 0) rd.ahead = rd.fetch(0);
       // Profile of this lane's 16 rows, as in the int16x2 warp fill.
       {

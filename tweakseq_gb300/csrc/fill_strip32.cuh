@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(32) fill_strip32_kernel(const FillArgs A) {
       uint64_t *row = A.strip_rows + A.strip_row_off[q];
       const uint32_t tag = strip_tag(strip);
       const bool hands_down = strip + 1 < strips;
-      StripReader<C> rd(row, strip_tag(strip - 1), n, t, A.spin_limit);
+      StripReader<C> rd{row, strip_tag(strip - 1), n, t, A.spin_limit > 0 ? A.spin_limit : kStripPolls, false, 0u};
       // Columns [C * chunk, C * chunk + C) of the top row go to the ring.
       auto take = [&](int chunk) {
         const int col = C * chunk + t;
