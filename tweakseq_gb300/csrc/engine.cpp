@@ -906,7 +906,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
   // 44-bit key, sorted by a stable LSD radix sort (O(n): the plan of an
   // 8M-pair batch must not cost seconds).
   ShapeChooser ch;
-  ch.out_mode = b->out_mode;
+  ch.out_mode = b->fill_mode;  // (tuned entries are those of the kernels that run)
   ch.local = b->local;
   ch.sms = sms;
   // Shapes follow the whole call's size (a chunk's pairs get the lane widths
@@ -963,7 +963,7 @@ int plan_impl(tsq_batch *b, const tsq_batch *owner, const uint8_t *seqs, int64_t
         // A tuned table may prefer int32 over int16x2 for this length bucket,
         // or the long pairs' fill for its int32 pairs.
         TunedChoice tc;
-        const bool tuned = ch.use_table && !ch.force.shape && tune_table_pick(b->out_mode, pd.a_len, pd.b_len, &tc);
+        const bool tuned = ch.use_table && !ch.force.shape && tune_table_pick(b->fill_mode, pd.a_len, pd.b_len, &tc);
         if (try16 && !(tuned && tc.sh.i16 == 0)) {
           const Range16 r16 = range16(p, sc, pd.a_len, pd.b_len);
           if (r16.lower) lt = (r16.upper && p->lane == TSQ_LANE_AUTO) ? 1 : 2;

@@ -11,7 +11,9 @@
 //     one pair over many warps; identity: a CTA of 8 warps) against one pair
 //     per warp group.
 // The table is written as JSON and read back by tsq_tune_load; batches
-// created with opts.autotune consult it.  Few-pair batches still get at
+// created with opts.autotune consult it.  Entries belong to the fill that
+// was timed: identity output that runs on traceback planes takes the alignment
+// entries.  Few-pair batches still get at
 // least enough lanes per pair to keep every SM busy (the planner takes the
 // larger of the tuned and the occupancy G), and a pair too long for any
 // warp group keeps the long pairs' fill whatever the table says.
@@ -192,6 +194,9 @@ extern "C" int tsq_tune_run(const char *json_path, int32_t quick) {
         tsq_batch_opts o{};
         o.device = dev;
         p.lane = cand.i16 ? TSQ_LANE_AUTO : TSQ_LANE_I32;
+        // Identity entries are for the fills that carry the counts; on traceback
+        // planes identity follows the alignment entries.
+        b.identity_planes_allowed = false;
         b.tune_force.shape = !cand.free;
         b.tune_force.sh = Shape{cand.G, 8, 0};
         b.tune_force.cta = cand.cta != 0;
