@@ -133,9 +133,9 @@ __global__ void __launch_bounds__(kCountThreads) consensus_count_kernel(const ui
 // 8.  All blocks of a row range run at the same time, so that the sectors that
 // two tiles share come from L2 once read.  It waits on its loads (with 16 rows
 // at once and none ahead 2 us more).
-// All launches of one call, before and after: 100,003 x 2,000 84 -> 61 us (200 MB,
-// 4.5 TB/s while counting; a plain copy reads and writes 6.8), 50,000 x 1,000
-// 63 -> 28, 10,000 x 1,000 58 -> 22.  Zeroing and folding cost about 5 us, so
+// All launches of one call, before and after: 100,000 x 2,000 with the L2 flushed
+// 86 -> 65 to 67 us (200 MB, 3.0 TB/s; a plain copy reads and writes 6.8), one call
+// after another 81 -> 53; 50,000 x 1,000 63 -> 28, 10,000 x 1,000 58 -> 22.  Zeroing and folding cost about 5 us, so
 // below kPairBytes the kernel above is the better one: 2,000 x 1,000 21.0 and
 // 20.9 us, 1,000 x 1,000 15.9 and 22.3.
 constexpr int kPairWarps = 32;

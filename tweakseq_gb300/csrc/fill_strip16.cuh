@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(32) fill_strip16_kernel(const FillArgs A) {
           const uint8_t *codeA = code_ring + ((cA0 + s0) & (kCodeRing16 - 1));
           const uint8_t *codeB = code_ring + ((cB0 + s0) & (kCodeRing16 - 1));
           const uint32_t *topp = top_ring + ((s0 & (kTopRing - 1)) + 1);
-        uint32_t *outp = out_ring + (s0 & (2 * C - 1));
+          uint32_t *outp = out_ring + (s0 & (2 * C - 1));
           step(s0, IntTag<0>{}, BoolTag<true>{}, BoolTag<false>{}, codeA, codeB, topp, outp);
           step(s0 + 1, IntTag<1>{}, BoolTag<true>{}, BoolTag<true>{}, codeA, codeB, topp, outp);
         };

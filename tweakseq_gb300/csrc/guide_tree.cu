@@ -296,8 +296,9 @@ __global__ void __launch_bounds__(kTreeThreads) tree_join_kernel(TreeArgs A, int
 // a full copy, and meet at hardware cluster barriers: 4.4 us a join at 500
 // leaves and 7.3 at 2,003 (NJ), of which about half are the three trips to L2
 // and the two barriers.  (Whole calls, before and now: 2,003 leaves NJ 31.2 and
-// 14.5 ms, 4,000 leaves UPGMA 90 and 43 ms; 8 CTAs for 16: 2,003 leaves NJ 20.8
-// for 16.2 ms; 512 threads for 256: 500 leaves 2.99 for 2.66 ms.)
+// 14.6 ms; 4,000 leaves, whose first 700 joins take two launches each, UPGMA 91 and
+// 56 to 59 ms, NJ 94 and 77 ms; 8 CTAs for 16: 2,003 leaves NJ 20.8 for 16.2 ms;
+// 512 threads for 256: 500 leaves 2.99 for 2.66 ms.)
 //
 // Rows, not the triangle.  Each slot keeps a lower bound of the criterion over
 // its whole row and a neighbour whose criterion is known exactly.  The smallest

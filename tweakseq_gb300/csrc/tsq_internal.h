@@ -75,10 +75,6 @@ struct Shape {
   int G, R, i16;
 };
 
-// A warp task: up to 32/G pairs of one lane width G, processed by one warp
-// (x = first index into the task list, y = (G << 16) | number of pairs).
-// The planner orders warp tasks longest first; warps of one persistent
-// launch pull them from a single counter.
 // What the strips of one pair leave for the one that finishes last.
 struct StripCtl {
   uint64_t key;     // local maximum as (score, -row, -column)
@@ -89,6 +85,10 @@ struct StripCtl {
 };
 static_assert(sizeof(StripCtl) == 32, "record size");
 
+// A warp task: up to 32/G pairs of one lane width G, processed by one warp
+// (x = first index into the task list, y = (G << 16) | number of pairs).
+// The planner orders warp tasks longest first; warps of one persistent
+// launch pull them from a single counter.
 struct FillArgs {
   const uint8_t *codes;
   const PairDev *pairs;
