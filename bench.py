@@ -929,7 +929,7 @@ def msa_leg(cpu_cols=40, cpu_tree_leaves=1000):
             cpu_s = time.perf_counter() - t0
             out[f"guide_tree_{method}_{n}"] = {
                 "ms": tree_ms, "joins": n - 1, "bitexact_vs_oracle": bool(same),
-                "what": "from the batch's device-resident identities: distances, n-1 join launches, joins to host",
+                "what": "from the batch's device-resident identities: distances, joins (one launch from 3,300 clusters down), joins to host",
                 "cpu_oracle_s_at_1000_leaves": cpu_s,
                 "cpu_oracle_s_extrapolated": cpu_s * (n / k) ** 3}
     return out
