@@ -165,12 +165,20 @@ int64_t tsq_results_strings(const tsq_result *r, int64_t n, char *buf, int64_t b
 /* Aligns n pairs over one host residue buffer in one planned launch
  * sequence (length buckets, persistent kernels, optional CUDA graph).
  * out[k] receives pair k.  Returns TSQ_E_INVALID_RESIDUE if any pair holds
- * an invalid residue (that pair's status says so; the others are valid). */
+ * an invalid residue (that pair's status says so; the others are valid).
+ *
+ * Device memory: alignment output, and identity output where it pays, keep
+ * traceback planes of about m*n/2 bytes a pair.  Identity output takes them up to
+ * 24 GB and a quarter of the memory that is free, and does without beyond that.
+ * The calling thread's cached engine keeps them for its next call; its other
+ * calls get them back when they need the memory. */
 int tsq_align_batch(const uint8_t *seqs, int64_t seqs_len,
                     const tsq_pair_desc *pairs, int64_t n, const tsq_params *p,
                     const tsq_batch_opts *opts, tsq_result *out);
 
-/* Device-resident batch: upload and plan once, run many times, read back. */
+/* Device-resident batch: upload and plan once, run many times, read back.  The
+ * object holds its device memory, traceback planes among it (see above), until it
+ * is destroyed. */
 typedef struct tsq_batch tsq_batch;
 int tsq_batch_create(const uint8_t *seqs, int64_t seqs_len,
                      const tsq_pair_desc *pairs, int64_t n, const tsq_params *p,
@@ -193,7 +201,7 @@ void tsq_batch_destroy(tsq_batch *b);
  * pairs, any parameters) are queued by tsq_server_submit from any thread; a
  * scheduler thread groups waiting requests with equal parameters into
  * ticks, admits a tick only while its device memory (residues, pair table,
- * results, band-boundary rows and, for alignments, traceback planes) fits
+ * results, boundary and strip rows and, for alignments, traceback planes) fits
  * the HBM budget left by the ticks in flight, and runs up to `slots` ticks
  * at once on separate streams.  Each request's results equal those of
  * tsq_align_batch on that request alone.
